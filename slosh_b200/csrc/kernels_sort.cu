@@ -177,13 +177,33 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* s_warp
     return ex;
 }
 
+// A thread's SCAN_ITEMS consecutive words as four 16-byte accesses where the tile is whole and both arrays start on 16
+// bytes (a caller's offset array may not), else word by word: the words of a warp's threads are 64 bytes apart, so
+// word accesses touch 16 lines each (4.1 M words: k_scan_down 25.9 us, 8.8 in
+// 16-byte accesses).
+__device__ __forceinline__ bool scan_vec(const uint32_t* in, const uint32_t* out, uint32_t base, uint32_t n) {
+    return ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0u && base + uint32_t(SCAN_ITEMS) <= n;
+}
+__device__ __forceinline__ void scan_load(const uint32_t* in, uint32_t base, uint32_t n, bool vec, uint32_t (&v)[SCAN_ITEMS]) {
+    if (vec) {
+#pragma unroll
+        for (int k = 0; k < SCAN_ITEMS / 4; ++k) {
+            const uint4 q = reinterpret_cast<const uint4*>(in + base)[k];
+            v[4 * k] = q.x; v[4 * k + 1] = q.y; v[4 * k + 2] = q.z; v[4 * k + 3] = q.w;
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < SCAN_ITEMS; ++k) v[k] = base + uint32_t(k) < n ? in[base + uint32_t(k)] : 0u;
+    }
+}
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan_reduce(const uint32_t* __restrict__ in, uint32_t n, uint32_t* __restrict__ sums) {
     __shared__ uint32_t s_warp[33];
     const uint32_t base = blockIdx.x * uint32_t(SCAN_TILE) + threadIdx.x * uint32_t(SCAN_ITEMS);
+    uint32_t vals[SCAN_ITEMS];
+    scan_load(in, base, n, scan_vec(in, in, base, n), vals);
     uint32_t v = 0u;
 #pragma unroll
-    for (int k = 0; k < SCAN_ITEMS; ++k)
-        if (base + uint32_t(k) < n) v += in[base + uint32_t(k)];
+    for (int k = 0; k < SCAN_ITEMS; ++k) v += vals[k];
     uint32_t total;
     block_excl_scan(v, s_warp, &total);
     if (threadIdx.x == 0) sums[blockIdx.x] = total;
@@ -206,18 +226,27 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_down(const uint32_t* in, 
     __shared__ uint32_t s_warp[33];
     const uint32_t base = blockIdx.x * uint32_t(SCAN_TILE) + threadIdx.x * uint32_t(SCAN_ITEMS);
     uint32_t vals[SCAN_ITEMS];
+    const bool vec = scan_vec(in, out, base, n);
+    scan_load(in, base, n, vec, vals);
     uint32_t v = 0u;
 #pragma unroll
-    for (int k = 0; k < SCAN_ITEMS; ++k) {
-        vals[k] = base + uint32_t(k) < n ? in[base + uint32_t(k)] : 0u;
-        v += vals[k];
-    }
+    for (int k = 0; k < SCAN_ITEMS; ++k) v += vals[k];
     uint32_t total;
     uint32_t run = block_excl_scan(v, s_warp, &total) + sums[blockIdx.x];
 #pragma unroll
     for (int k = 0; k < SCAN_ITEMS; ++k) {
-        if (base + uint32_t(k) < n) out[base + uint32_t(k)] = run;
-        run += vals[k];
+        const uint32_t t = vals[k];
+        vals[k] = run;
+        run += t;
+    }
+    if (vec) {
+#pragma unroll
+        for (int k = 0; k < SCAN_ITEMS / 4; ++k)
+            reinterpret_cast<uint4*>(out + base)[k] = make_uint4(vals[4 * k], vals[4 * k + 1], vals[4 * k + 2], vals[4 * k + 3]);
+    } else {
+#pragma unroll
+        for (int k = 0; k < SCAN_ITEMS; ++k)
+            if (base + uint32_t(k) < n) out[base + uint32_t(k)] = vals[k];
     }
 }
 
