@@ -860,8 +860,9 @@ struct Ctx {
                 else mgpcg(pressure, divergence, S.pcg_iterations, 0.0f, 0, coarse, 0);
             } else {
                 const float omega = clampf_h(S.sor_weight, 0.5f, 1.95f);
+                count(launch_rbgs_words(d, mg, shape, stream));
                 for (int it = 0; it < S.pressure_iterations; ++it)
-                    for (uint32_t colour = 0; colour < 2u; ++colour) count(launch_rbgs(d, pressure, divergence, colour, omega, shape, stream));
+                    for (uint32_t colour = 0; colour < 2u; ++colour) count(launch_rbgs(d, mg, pressure, divergence, colour, omega, shape, stream));
                 last_iterations = S.pressure_iterations;
                 last_converged = true;
             }
@@ -882,7 +883,7 @@ struct Ctx {
             } else {
                 for (int it = 0; it < std::max(S.density_projection_iterations, 1); ++it)
                     for (uint32_t colour = 0; colour < 2u; ++colour)
-                        count(launch_rbgs(d, density_q, density_rhs, colour, 1.7f, shape, stream));
+                        count(launch_rbgs(d, mg, density_q, density_rhs, colour, 1.7f, shape, stream));
             }
         }
         {

@@ -47,7 +47,6 @@ int launch_mark_cells(const Dev& d, const Pass& p, const Shape& sh, cudaStream_t
 int launch_normalize_faces(const Dev& d, const Pass& p, float* vel, const Shape& sh, cudaStream_t s);
 int launch_viscosity(const Dev& d, const Pass& p, const float* ustar, const float* src, float* dst, const Shape& sh, cudaStream_t s);
 int launch_divergence(const Dev& d, const Pass& p, const float* vel, const Shape& sh, cudaStream_t s);
-int launch_rbgs(const Dev& d, float* pres, const float* rhs, uint32_t parity, float omega, const Shape& sh, cudaStream_t s);
 int launch_project(const Dev& d, const Pass& p, float* vel, const Shape& sh, cudaStream_t s);
 int launch_residual(const Dev& d, const Pass& p, const float* vel, const Shape& sh, cudaStream_t s);
 // Two-way collider coupling after the projection (wetted faces, binary force, seepage contacts and, with
@@ -150,6 +149,10 @@ int launch_mg_coarse_setup(const Dev& d, const MGState& m, const Shape& sh, cuda
 // handle: the WHILE node's condition when the solve runs as a CUDA graph, 0 otherwise.
 int launch_pcg_init(const Dev& d, const MGState& m, const float* p, const float* div, unsigned long long handle, const Shape& sh,
                     cudaStream_t s, bool words = true);
+// Red-black SOR (PressureRBGSCS): the stencil words and neighbour slots of this substep's cell types (once for both its
+// solves), then one launch per colour sweep.
+int launch_rbgs_words(const Dev& d, const MGState& m, const Shape& sh, cudaStream_t s);
+int launch_rbgs(const Dev& d, const MGState& m, float* pres, const float* rhs, uint32_t parity, float omega, const Shape& sh, cudaStream_t s);
 int launch_vcycle(const Dev& d, const MGState& m, int coarse_iterations, const Shape& sh, cudaStream_t s);
 int launch_pcg_apply_a(const Dev& d, const MGState& m, const Shape& sh, cudaStream_t s);
 int launch_pcg_update_pr(const Dev& d, const MGState& m, float* p, unsigned long long handle, const Shape& sh, cudaStream_t s);

@@ -3,8 +3,7 @@
 // Reference kernels (PLUG/Shaders/Private/Slosh.usf): BrickFreeCS / BrickAllocCS / PoolArgsCS
 // (:1719-1817), ClearNewSlotsCS (:1819-1831), BuildSolidCS (:365-395) fused into MarkCellsCS
 // (:569-598), NormalizeFace (:604-651), ViscosityJacobiFace (:657-686), DivergenceCS (:692-741),
-// DensityProjectionRhsCS (:775-805), DensityDisplacementFace (:808-828), PressureRBGSCS (:860-892),
-// ProjectFace (:995-1052), ResidualCS (:1222-1257), ExtrapolateFace (:1263-1310).
+// DensityProjectionRhsCS (:775-805), DensityDisplacementFace (:808-828), ProjectFace (:995-1052), ResidualCS (:1222-1257), ExtrapolateFace (:1263-1310).
 //
 // Every brick pass is a grid-stride loop of 256-thread CTAs over the active-brick list; thread t of a
 // CTA owns cells t and t + 256 of the current brick, so each warp touches 32 consecutive cells of a
@@ -460,29 +459,6 @@ __global__ void __launch_bounds__(GRID_THREADS) k_divergence(Dev d, Pass p, cons
     });
 }
 
-// ---- PressureRBGSCS: one SOR colour sweep ----------------------------------------------------------------
-__global__ void __launch_bounds__(GRID_THREADS) k_rbgs(Dev d, float* __restrict__ pres, const float* __restrict__ rhs,
-                                                       uint32_t parity, float omega) {
-    for_active_cells<false>(d, [&](uint32_t index, int3 c) {
-        if (type_of(d.cell_type[index]) != CELL_FLUID) return;
-        if ((uint32_t(c.x + c.y + c.z) & 1u) != parity) return;
-        float sum = 0.0f;
-        const float diag = d.cell_diag[index];
-#pragma unroll
-        for (int n = 0; n < 6; ++n) {
-            const int3 nb = add3(c, nbr_off(n));
-            if (!in_grid(d, nb)) continue;
-            const uint32_t ni = nbr_at<false>(d, index, c, n);
-            if (type_of(d.cell_type[ni]) == CELL_FLUID) sum = sum + pres[ni];
-        }
-        if (diag > 0.0f) {
-            const float gs = (sum - rhs[index]) / diag;
-            const float old = pres[index];
-            pres[index] = old + omega * (gs - old);
-        }
-    });
-}
-
 // ---- ProjectFace (its two-way coupling terms are accumulated by k_coupling_faces after the pass) ---------
 // Every value a face may need (the neighbour's type and pressure, the cell's pressure, the face's velocity
 // and flags) is loaded before the types are tested, so a cell costs one round of loads; a neighbour outside
@@ -895,10 +871,6 @@ int launch_viscosity(const Dev& d, const Pass& p, const float* ustar, const floa
 }
 int launch_divergence(const Dev& d, const Pass& p, const float* vel, const Shape& sh, cudaStream_t s) {
     k_divergence<<<sh.brick_ctas, GRID_THREADS, 0, s>>>(d, p, vel);
-    return 1;
-}
-int launch_rbgs(const Dev& d, float* pres, const float* rhs, uint32_t parity, float omega, const Shape& sh, cudaStream_t s) {
-    k_rbgs<<<sh.brick_ctas, GRID_THREADS, 0, s>>>(d, pres, rhs, parity, omega);
     return 1;
 }
 int launch_project(const Dev& d, const Pass& p, float* vel, const Shape& sh, cudaStream_t s) {

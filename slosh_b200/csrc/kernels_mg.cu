@@ -401,6 +401,57 @@ __device__ __forceinline__ void w0_black(const Dev& d, const MGState& m, Prep pr
     }
 }
 
+// ---- PressureRBGSCS: one SOR colour sweep ----------------------------------------------------------------
+// Reference: PLUG/Shaders/Private/Slosh.usf:860-892. The cells of one colour (parity 0: red) of every active brick, one
+// warp per brick, 8 cells per lane as in w0_black, with the per-solve stencil words and neighbour slots (k_pcg_words)
+// that the MGPCG passes use: all nine loads of four cells are in flight at once, where the sweep over cell types read
+// the brick table and the neighbour's type before each value. A colour's cells are read by other warps only through
+// the other colour's sweep, so reading and writing one array is safe.
+// Bound by L2 latency and bandwidth: 192^3 with 1.09 M fluid cells 23.3 us a colour before, 5.9 now (a frame of 200 + 30
+// iterations 11.8 -> 3.6 ms); 96x96x72 with 0.1 M fluid cells 8.8 -> 4.8 us. Half a brick per warp (one round of loads)
+// takes 1.25 instead of 1.41 ms for a frame of the small tank but 4.0 instead of 3.6 ms for the large one.
+__device__ __forceinline__ uint32_t colour_local(uint32_t lane, uint32_t k, uint32_t parity) {
+    const uint32_t y = lane >> 2;
+    return 2u * (lane & 3u) + ((y + k + parity) & 1u) + 8u * y + 64u * k;
+}
+__global__ void __launch_bounds__(GRID_THREADS) k_rbgs(Dev d, MGState m, float* pres, const float* __restrict__ rhs, uint32_t parity, float omega) {
+    pdl_entry();
+    constexpr uint32_t B = 4u;
+    const uint32_t active = d.active_bricks[0];
+    const uint32_t lane = threadIdx.x & 31u, wpb = blockDim.x >> 5;
+    for (uint32_t e = blockIdx.x * wpb + (threadIdx.x >> 5); e < active; e += gridDim.x * wpb) {
+        const uint4 s0 = *reinterpret_cast<const uint4*>(m.nbr_slots + 8u * e);
+        const uint4 s1 = *reinterpret_cast<const uint4*>(m.nbr_slots + 8u * e + 4u);
+        const uint32_t ns[6] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y};
+        const uint32_t base = s1.z * BRICK_CELLS;
+#pragma unroll
+        for (uint32_t k0 = 0; k0 < 8u; k0 += B) {
+            uint32_t w[B];
+            float b[B], dg[B], old[B], n[B][6];
+#pragma unroll
+            for (uint32_t j = 0; j < B; ++j) {
+                const uint32_t l = colour_local(lane, k0 + j, parity), i = base + l;
+                w[j] = m.word[i];
+                b[j] = rhs[i];
+                dg[j] = d.cell_diag[i];
+                old[j] = pres[i];
+#pragma unroll
+                for (int q = 0; q < 6; ++q) n[j][q] = pres[l0_nbr(i, l, q, ns)];
+            }
+#pragma unroll
+            for (uint32_t j = 0; j < B; ++j) {
+                if (!(w[j] & W_FLUID) || !(dg[j] > 0.0f)) continue;
+                float sum = 0.0f;
+#pragma unroll
+                for (int q = 0; q < 6; ++q)
+                    if ((w[j] >> q) & 1u) sum = sum + n[j][q];
+                const float gs = (sum - b[j]) / dg[j];
+                pres[base + colour_local(lane, k0 + j, parity)] = old[j] + omega * (gs - old[j]);
+            }
+        }
+    }
+}
+
 struct Nb6 {
     uint32_t w;
     float c0, c1, c2;
@@ -2266,6 +2317,14 @@ int launch_vcycle(const Dev& d, const MGState& m, int coarse_iterations, const S
         n += 2;
     }
     return n;
+}
+int launch_rbgs_words(const Dev& d, const MGState& m, const Shape& sh, cudaStream_t s) {
+    launch_k(k_pcg_words, sh.mg_ctas, GRID_THREADS, 0, s, d, m);
+    return 1;
+}
+int launch_rbgs(const Dev& d, const MGState& m, float* pres, const float* rhs, uint32_t parity, float omega, const Shape& sh, cudaStream_t s) {
+    launch_k(k_rbgs, sh.mg_ctas, GRID_THREADS, 0, s, d, m, pres, rhs, parity, omega);
+    return 1;
 }
 int launch_pcg_apply_a(const Dev& d, const MGState& m, const Shape& sh, cudaStream_t s) {
     if (mg_staged()) ST_LAUNCH(k_apply_a_st, 2, 1, d, m, sh, s);
