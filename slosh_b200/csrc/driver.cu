@@ -172,6 +172,8 @@ struct Ctx {
     SortBuffers sortb{};
     P2GGather gather{};  // the per-cell particle index of the gather P2G (allocated only when it is on)
     MGState mg{};
+    int cluster_ctas = 0;          // CTAs of the cluster form of the solve (0: not available for this layout)
+    uint32_t bricks_estimate = 0;  // active bricks of the last frame; the layout's most before the first
 
     // pinned host staging
     slosh_collider_t* h_colliders = nullptr;
@@ -456,6 +458,8 @@ struct Ctx {
         total_emitted = 0;
         prev_dt = 0.0f;
         last_max_speed = 0.0f;
+        cluster_ctas = mg_solve_cluster(mg);
+        bricks_estimate = num_pool_bricks - 1u;
         shape.num_sms = num_sms;
         shape.brick_ctas = brick_ctas_for(ctas_per_sm);
         shape.mg_ctas = brick_ctas_for(mg_ctas_per_sm);
@@ -710,8 +714,11 @@ struct Ctx {
         const bool tol_mode = fixed_iterations <= 0;
         const uint32_t limit = tol_mode ? uint32_t(std::max(max_iterations, 1)) : uint32_t(std::min(std::max(fixed_iterations, 1), 100));
         const Dev d = dev();
+        // few active bricks: the whole solve in one cluster (the form does not change the result, so the last frame's
+        // count, which the host has, is enough to choose by)
+        const bool cluster = cluster_ctas > 0 && bricks_estimate <= mg_solve_cluster_bricks();
         SolveGraph* G = nullptr;
-        if (use_graphs) {
+        if (use_graphs && !cluster) {
             try {
                 G = solve_graph(p, div, limit, tol_mode, tolerance, coarse_iterations, slot == 0);
             } catch (const CudaError& e) {
@@ -721,7 +728,10 @@ struct Ctx {
                 destroy_graphs();
             }
         }
-        if (G) {
+        if (cluster) {
+            const int n = launch_solve_cluster(d, mg, cluster_ctas, p, div, limit, tol_mode, double(tolerance), coarse_iterations, slot == 0, stream);
+            frame_solves.push_back({n, 0, slot});
+        } else if (G) {
             CK(cudaGraphLaunch(G->exec, stream));
             frame_solves.push_back({G->pre_nodes, G->body_nodes, slot});
         } else {
@@ -934,6 +944,7 @@ void Ctx::end_frame_enqueue() {
 void Ctx::end_frame_finish() {
     CK(cudaStreamSynchronize(stream));
     if (substeps > 0) {
+        bricks_estimate = h_stats[7];
         float ms;
         std::memcpy(&ms, &h_stats[0], 4);
         last_max_speed = std::isfinite(ms) ? ms : 0.0f;

@@ -66,12 +66,14 @@ __device__ __forceinline__ void lv_st(float* a, uint32_t i, uint32_t prec, float
 // two that brings the level-0 residual's norm (||r||^2 in scalars[5] when a V-cycle starts) to about 1, and the
 // prolongation back to level 0 divides by it, so FP16's narrow exponent range holds the coarse values without
 // flushing small ones; the V-cycle is linear and a power of two scales exactly. 1 with FP32 storage.
-__device__ __forceinline__ float coarse_scale(const MGState& m) {
+__device__ __forceinline__ float coarse_scale(const MGState& m, double rr) {
     if (m.lv[1].prec == SLOSH_PRECISION_FP32) return 1.0f;
-    const double rr = m.scalars[5];
     int e = rr > 0.0 ? -ilogb(sqrt(rr)) : 0;
     e = max(-60, min(60, e));
     return ldexpf(1.0f, e);
+}
+__device__ __forceinline__ float coarse_scale(const MGState& m) {
+    return m.lv[1].prec == SLOSH_PRECISION_FP32 ? 1.0f : coarse_scale(m, m.scalars[5]);
 }
 // Coarse-level stencil word bits (k_level_words): bits 0-5 fluid neighbour, 6 fluid, 7 red, 8-13 non-solid neighbour.
 constexpr uint32_t CW_FLUID = 1u << 6, CW_RED = 1u << 7, CW_NONSOLID_SHIFT = 8u;
@@ -179,6 +181,19 @@ __device__ double final_reduce(const double* partials, uint32_t n, DotSmem& sm) 
     return total;
 }
 
+// The warp's and the thread's place in a pass. Passes launched over the whole GPU give a CTA consecutive entries
+// (neighbouring bricks share its L1); in the cluster solve (CL), whose few bricks do not fill its warps, they are dealt
+// out over the CTAs, so every SM's loads and issue slots are used.
+template <bool CL>
+__device__ __forceinline__ uint32_t pass_warp() {
+    const uint32_t w = threadIdx.x >> 5;
+    return CL ? w * gridDim.x + blockIdx.x : blockIdx.x * (blockDim.x >> 5) + w;
+}
+template <bool CL>
+__device__ __forceinline__ uint32_t pass_thread() {
+    return CL ? pass_warp<true>() * 32u + (threadIdx.x & 31u) : blockIdx.x * blockDim.x + threadIdx.x;
+}
+
 // Visits the cells of level l (1..3) that lie in the active bricks' footprints: fn(ci, c). Levels
 // whose cells are coarser than a brick are scanned densely.
 // Thread t0 of `stride` threads takes footprint cells t0, t0 + stride, ...
@@ -207,12 +222,12 @@ __device__ __forceinline__ void for_footprint_span(const Dev& d, const MGLevel& 
 // footprints have an even side, so a cell's colour is that of its position inside the footprint: item j of a brick
 // is (2 (j mod s/2) + ((y + z + parity) & 1), y, z) with y = (j / (s/2)) mod s, z = j / (s^2/2). A sweep then
 // visits only the cells it updates: half the threads of the all-cell walk.
-template <class Fn>
+template <bool CL = false, class Fn>
 __device__ __forceinline__ void for_footprint_colour(const Dev& d, const MGLevel& L, int l, uint32_t parity, Fn fn) {
     const uint32_t side = uint32_t(8 >> l), half = side / 2u;
     const uint32_t per = side * side * half;
     const uint32_t count = d.active_bricks[0];
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;; t += gridDim.x * blockDim.x) {
+    for (uint32_t t = pass_thread<CL>();; t += gridDim.x * blockDim.x) {
         const uint32_t e = t / per, j = t % per;
         const uint32_t brick = d.active_bricks[1u + min(e, d.num_bricks - 1u)];
         if (e >= count) break;
@@ -223,9 +238,9 @@ __device__ __forceinline__ void for_footprint_colour(const Dev& d, const MGLevel
         if (inside3(c, L.dim)) fn(lin3(c, L.dim), c);
     }
 }
-template <class Fn>
+template <bool CL = false, class Fn>
 __device__ __forceinline__ void for_footprint(const Dev& d, const MGLevel& L, int l, Fn fn) {
-    for_footprint_span(d, L, l, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, fn);
+    for_footprint_span(d, L, l, pass_thread<CL>(), gridDim.x * blockDim.x, fn);
 }
 
 // ---- level-0 stencil words ------------------------------------------------------------------------
@@ -312,13 +327,14 @@ __device__ __forceinline__ void nbrs6(const Q6& q, const X2& x, uint32_t h, int 
 // load(g, ns) gathers a round's values; apply(g, vals, v0[4], v1[4]) computes and stores one round and
 // yields the cells' dot terms. The loads of B rounds are issued before any of them is applied. With
 // NDOT > 0 the last CTA reduces the brick partials (canonical tree) and calls store(t0, t1) in thread 0.
-template <int NDOT, int B, class Load, class Apply, class Store>
-__device__ __forceinline__ void w4_pass(const Dev& d, const MGState& m, uint32_t counter, Load load, Apply apply, Store store) {
-    __shared__ DotSmem sm;
+// CL (the cluster solve): the pass ends with the brick partials stored, and its caller reduces them.
+template <int NDOT, int B, bool CL = false, class Load, class Apply, class Store>
+__device__ __forceinline__ void w4_pass(const Dev& d, const MGState& m, uint32_t counter, Load load, Apply apply, Store store,
+                                        uint32_t first_partial = 0u) {
     const uint32_t active = d.active_bricks[0];
     const uint32_t cap = d.num_pool_bricks;
     const uint32_t lane = threadIdx.x & 31u, wpb = blockDim.x >> 5;
-    for (uint32_t e = blockIdx.x * wpb + (threadIdx.x >> 5); e < active; e += gridDim.x * wpb) {
+    for (uint32_t e = pass_warp<CL>(); e < active; e += gridDim.x * wpb) {
         const uint4 s0 = *reinterpret_cast<const uint4*>(m.nbr_slots + 8u * e);
         const uint4 s1 = *reinterpret_cast<const uint4*>(m.nbr_slots + 8u * e + 4u);
         const uint32_t ns[6] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y};
@@ -342,14 +358,16 @@ __device__ __forceinline__ void w4_pass(const Dev& d, const MGState& m, uint32_t
         }
         if (NDOT > 0) {
             const double t0 = warp_fold(acc0);
-            if (lane == 0) m.partials[e] = t0;
+            if (lane == 0) m.partials[first_partial + e] = t0;
         }
         if (NDOT > 1) {
             const double t1 = warp_fold(acc1);
             if (lane == 0) m.partials[cap + e] = t1;
         }
     }
-    if (NDOT == 0) return;
+    if constexpr (NDOT == 0 || CL) return;
+    else {
+    __shared__ DotSmem sm;
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) sm.last = (atomicAdd(m.counters + counter, 1u) == gridDim.x - 1u) ? 1u : 0u;
@@ -365,6 +383,7 @@ __device__ __forceinline__ void w4_pass(const Dev& d, const MGState& m, uint32_t
             m.counters[counter] = 0u;
         }
     }
+    }
 }
 
 // The 256 black cells ((x + y + z) odd) of every active brick, one warp per brick, 8 cells per lane:
@@ -375,11 +394,11 @@ __device__ __forceinline__ uint32_t black_local(uint32_t lane, uint32_t k) {
     const uint32_t y = lane >> 2;
     return 2u * (lane & 3u) + ((y + k + 1u) & 1u) + 8u * y + 64u * k;
 }
-template <int B, class Prep, class Load, class Apply>
+template <int B, bool CL, class Prep, class Load, class Apply>
 __device__ __forceinline__ void w0_black(const Dev& d, const MGState& m, Prep prep, Load load, Apply apply) {
     const uint32_t active = d.active_bricks[0];
     const uint32_t lane = threadIdx.x & 31u, wpb = blockDim.x >> 5;
-    for (uint32_t e = blockIdx.x * wpb + (threadIdx.x >> 5); e < active; e += gridDim.x * wpb) {
+    for (uint32_t e = pass_warp<CL>(); e < active; e += gridDim.x * wpb) {
         const uint4 s0 = *reinterpret_cast<const uint4*>(m.nbr_slots + 8u * e);
         const uint4 s1 = *reinterpret_cast<const uint4*>(m.nbr_slots + 8u * e + 4u);
         const uint32_t ns[6] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y};
@@ -474,9 +493,10 @@ struct SweepQ {
 };
 // PROLONGED (the first red sweep after k_prolong_smooth0 with an over-relaxed smoother): the red cells' stored
 // z lacks the prolongation, which the fused kernel adds only to the values it reads, so the sweep rebuilds each
-// red cell's prolonged value z + x_parent / coarse scale (fluid parents) from level 1, as k_prolong_smooth0 does.
+// red cell's prolonged value z + x_parent / coarse scale (ivs: its reciprocal, a power of two; fluid parents) from
+// level 1, as k_prolong_smooth0 does.
 template <bool PROLONGED = false>
-__device__ __forceinline__ SweepQ load_sweep(const Dev& d, const MGState& m, const Geo& g, const uint32_t* ns) {
+__device__ __forceinline__ SweepQ load_sweep(const Dev& d, const MGState& m, const Geo& g, const uint32_t* ns, float ivs = 1.0f) {
     SweepQ v;
     v.z = load_q6(m.z, g, ns);
     v.r = ld4(m.r + g.i);
@@ -485,7 +505,6 @@ __device__ __forceinline__ SweepQ load_sweep(const Dev& d, const MGState& m, con
     v.pa = v.pb = 0.0f;
     if (PROLONGED) {
         const MGLevel C = m.lv[1];
-        const float ivs = 1.0f / coarse_scale(m);  // a power of two: exact
         const int3 bc = brick_coord_of(d, g.b);
         float pv[2];
 #pragma unroll
@@ -550,11 +569,11 @@ __global__ void k_build_type_fp(Dev d, MGLevel fine, MGLevel coarse, int lc) {
 // x = t & 7, y = (t >> 3) + 4 (k & 1), z = k >> 1, so the children of one coarse cell are combined across lanes
 // t ^ 1, t ^ 2, t ^ 4 (x), t ^ 8, t ^ 16 and k ^ 1 (y), k ^ 2, k ^ 4, k ^ 8 (z).
 __device__ __forceinline__ uint32_t type_of_flags(uint32_t f) { return (f & 1u) ? CELL_AIR : ((f & 2u) ? CELL_FLUID : CELL_SOLID); }
-__global__ void __launch_bounds__(256) k_build_types_fp13(Dev d, MGState m, int top) {
-    pdl_entry();
+template <bool CL>
+__device__ __forceinline__ void build_types_fp13(const Dev& d, const MGState& m, int top) {
     const uint32_t active = d.active_bricks[0];
     const uint32_t lane = threadIdx.x & 31u, wpb = blockDim.x >> 5;
-    for (uint32_t e = blockIdx.x * wpb + (threadIdx.x >> 5); e < active; e += gridDim.x * wpb) {
+    for (uint32_t e = pass_warp<CL>(); e < active; e += gridDim.x * wpb) {
         const uint32_t brick = d.active_bricks[1u + e];
         const uint32_t slot = __ldg(d.brick_table + brick);
         const int3 bc = brick_coord_of(d, brick);
@@ -603,8 +622,10 @@ __global__ void __launch_bounds__(256) k_build_types_fp13(Dev d, MGState m, int 
         if (lane == 0u && inside3(bc, L.dim)) L.type[lin3(bc, L.dim)] = type_of_flags(v);
     }
 }
-// The words of levels 1 to top (top <= 3) in one launch: each thread walks the three footprints in turn.
-__global__ void k_level_words_fp13(Dev d, MGState m, int top);
+__global__ void __launch_bounds__(256) k_build_types_fp13(Dev d, MGState m, int top) {
+    pdl_entry();
+    build_types_fp13<false>(d, m, top);
+}
 
 // ---- coarse-level stencil words (once per solve, after the coarse types) -----------------------------------
 
@@ -632,13 +653,18 @@ __global__ void k_level_words_fp(Dev d, MGLevel L, int l) {
     pdl_entry();
     for_footprint(d, L, l, [&](uint32_t i, int3 c) { level_word_cell(L, i, c); });
 }
-__global__ void k_level_words_fp13(Dev d, MGState m, int top) {
-    pdl_entry();
-    const uint32_t t0 = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+// The words of levels 1 to top (top <= 3) in one launch: each thread walks the three footprints in turn.
+template <bool CL>
+__device__ __forceinline__ void level_words_fp13(const Dev& d, const MGState& m, int top) {
+    const uint32_t t0 = pass_thread<CL>(), stride = gridDim.x * blockDim.x;
     for (int l = 1; l <= top; ++l) {
         const MGLevel& L = m.lv[l];
         for_footprint_span(d, L, l, t0, stride, [&](uint32_t i, int3 c) { level_word_cell(L, i, c); });
     }
+}
+__global__ void k_level_words_fp13(Dev d, MGState m, int top) {
+    pdl_entry();
+    level_words_fp13<false>(d, m, top);
 }
 // DiagEpsilon plus one per non-solid neighbour, added in neighbour order like FINE_STENCIL.
 __device__ __forceinline__ float word_diag(uint32_t w) {
@@ -680,11 +706,11 @@ __device__ __forceinline__ float word_sum(const float* x, uint32_t w, uint32_t i
 // ---- PCGInitCS (+ ||r0||^2 and ||b||^2, and the decision whether any iteration runs) ----------------------
 // First stores the solve's stencil words and each active brick's neighbour and own slots; the residual
 // pass itself reads the cell types directly (its neighbours' words may not be written yet).
-__global__ void __launch_bounds__(GRID_THREADS) k_pcg_words(Dev d, MGState m) {
-    pdl_entry();
+template <bool CL>
+__device__ __forceinline__ void pcg_words(const Dev& d, const MGState& m) {
     const uint32_t active = d.active_bricks[0];
     const uint32_t lane = threadIdx.x & 31u, wpb = blockDim.x >> 5;
-    for (uint32_t e = blockIdx.x * wpb + (threadIdx.x >> 5); e < active; e += gridDim.x * wpb) {
+    for (uint32_t e = pass_warp<CL>(); e < active; e += gridDim.x * wpb) {
         const uint32_t brick = d.active_bricks[1u + e];
         const uint32_t slot = __ldg(d.brick_table + brick);
         const int3 bc = brick_coord_of(d, brick);
@@ -733,15 +759,18 @@ __global__ void __launch_bounds__(GRID_THREADS) k_pcg_words(Dev d, MGState m) {
         }
     }
 }
-__global__ void __launch_bounds__(GRID_THREADS) k_pcg_init(Dev d, MGState m, const float* __restrict__ p, const float* __restrict__ div,
-                                                           unsigned long long handle) {
+__global__ void __launch_bounds__(GRID_THREADS) k_pcg_words(Dev d, MGState m) {
     pdl_entry();
+    pcg_words<false>(d, m);
+}
+template <bool CL, class Store>
+__device__ __forceinline__ void pcg_init(const Dev& d, const MGState& m, const float* p, const float* div, Store store) {
     struct V {
         Q6 p;
         float4 dv, dg;
         uint32_t w;
     };
-    w4_pass<2, 1>(d, m, 0,
+    w4_pass<2, 1, CL>(d, m, 0,
         [&](const Geo& g, const uint32_t* ns) {
             V v;
             v.p = load_q6(p, g, ns);
@@ -772,14 +801,19 @@ __global__ void __launch_bounds__(GRID_THREADS) k_pcg_init(Dev d, MGState m, con
             st4(m.r + g.i, r);
             st4(m.z + g.i, z);
         },
-        [&](double rr, double bb) {
-            m.scalars[5] = rr;
-            m.scalars[4] = bb;
-            const double rel = bb > 0.0 ? sqrt(rr / bb) : 0.0;
-            const bool run = m.ctl[1] > 0u && !(m.ctl[2] != 0u && rel <= m.scalars[8]);
-            if (!run) m.ctl[3] = 1u;
-            if (handle) cudaGraphSetConditional(handle, run ? 1u : 0u);
-        });
+        store);
+}
+__global__ void __launch_bounds__(GRID_THREADS) k_pcg_init(Dev d, MGState m, const float* __restrict__ p, const float* __restrict__ div,
+                                                           unsigned long long handle) {
+    pdl_entry();
+    pcg_init<false>(d, m, p, div, [&](double rr, double bb) {
+        m.scalars[5] = rr;
+        m.scalars[4] = bb;
+        const double rel = bb > 0.0 ? sqrt(rr / bb) : 0.0;
+        const bool run = m.ctl[1] > 0u && !(m.ctl[2] != 0u && rel <= m.scalars[8]);
+        if (!run) m.ctl[3] = 1u;
+        if (handle) cudaGraphSetConditional(handle, run ? 1u : 0u);
+    });
 }
 
 // ---- MGSmoothCS on level 0 (z as x, r as b); with dot the r.z reduction shifts rho -----------------------
@@ -798,11 +832,10 @@ __device__ __forceinline__ Nb6 load_black(const Dev& d, const MGState& m, uint32
 // Red sweep; with DOT also rho = r . z over all cells (red: the new value, black: the current z), which
 // shifts rho. Cells the sweep does not update are stored back unchanged (each cell belongs to one warp's
 // brick).
-template <bool DOT, bool PROLONGED = false>
-__global__ void __launch_bounds__(GRID_THREADS, 3) k_smooth0(Dev d, MGState m) {
-    pdl_entry();
-    w4_pass<DOT ? 1 : 0, 1>(d, m, 1,
-        [&](const Geo& g, const uint32_t* ns) { return load_sweep<PROLONGED>(d, m, g, ns); },
+template <bool DOT, bool PROLONGED, bool CL>
+__device__ __forceinline__ void smooth0_red(const Dev& d, const MGState& m, float ivs) {
+    w4_pass<DOT ? 1 : 0, 1, CL>(d, m, 1,
+        [&](const Geo& g, const uint32_t* ns) { return load_sweep<PROLONGED>(d, m, g, ns, ivs); },
         [&](const Geo& g, const SweepQ& v, double* v0, double*) {
             const X2 x = partner(v.z);
             float out[4];
@@ -827,15 +860,26 @@ __global__ void __launch_bounds__(GRID_THREADS, 3) k_smooth0(Dev d, MGState m) {
         [&](double rho, double) { m.scalars[3] = m.scalars[0]; m.scalars[0] = rho; });
 }
 
-// Black sweep (no dot product).
-__global__ void __launch_bounds__(GRID_THREADS) k_smooth0_black(Dev d, MGState m) {
+template <bool DOT, bool PROLONGED = false>
+__global__ void __launch_bounds__(GRID_THREADS, 3) k_smooth0(Dev d, MGState m) {
     pdl_entry();
-    w0_black<4>(d, m, [](uint32_t, uint32_t) {},
+    smooth0_red<DOT, PROLONGED, false>(d, m, PROLONGED ? 1.0f / coarse_scale(m) : 1.0f);
+}
+
+// Black sweep (no dot product).
+template <bool CL>
+__device__ __forceinline__ void smooth0_black(const Dev& d, const MGState& m) {
+    w0_black<4, CL>(d, m, [](uint32_t, uint32_t) {},
         [&](uint32_t i, uint32_t l, const uint32_t* ns) { return load_black(d, m, i, l, ns); },
         [&](uint32_t i, uint32_t, const Nb6& v) {
             if (!(v.w & W_FLUID)) return;
             m.z[i] = relax0(m, v.c1, (v.c0 + nb_sum(v.n, v.w)) / (v.c2 + DIAG_EPSILON));
         });
+}
+
+__global__ void __launch_bounds__(GRID_THREADS) k_smooth0_black(Dev d, MGState m) {
+    pdl_entry();
+    smooth0_black<false>(d, m);
 }
 
 // ---- MGProlongCS (level 1 -> 0) fused with the following black sweep ------------------------------
@@ -845,14 +889,11 @@ __global__ void __launch_bounds__(GRID_THREADS) k_smooth0_black(Dev d, MGState m
 // stages the level-1 correction of its brick's 4^3 parents and their face neighbours (a 6^3 block,
 // x_c where the parent is fluid and 0 elsewhere) in shared memory. Adding +0 instead of skipping the
 // addition changes at most the sign of a zero z_n, which the neighbour sum (started at +0) absorbs.
-__global__ void __launch_bounds__(GRID_THREADS) k_prolong_smooth0(Dev d, MGState m) {
-    pdl_entry();
-    constexpr int WARPS = GRID_THREADS / 32;
-    __shared__ float s_cx[WARPS][216];
+// cx: the warp's 216 floats of shared memory; ivs: 1 / coarse scale, a power of two.
+template <bool CL>
+__device__ __forceinline__ void prolong_smooth0(const Dev& d, const MGState& m, float ivs, float* cx) {
     const MGLevel C = m.lv[1];
-    const float ivs = 1.0f / coarse_scale(m);  // a power of two: exact
-    float* cx = s_cx[threadIdx.x >> 5];
-    w0_black<4>(d, m,
+    w0_black<4, CL>(d, m,
         [&](uint32_t brick, uint32_t lane) {
             const int3 bc = brick_coord_of(d, brick);
             __syncwarp();
@@ -888,6 +929,12 @@ __global__ void __launch_bounds__(GRID_THREADS) k_prolong_smooth0(Dev d, MGState
                 if ((v.w >> n) & 1u) sum = sum + (v.n[n] + cx[po[n]]);
             m.z[i] = relax0(m, v.c1 + cx[p], (v.c0 + sum) / (v.c2 + DIAG_EPSILON));
         });
+}
+
+__global__ void __launch_bounds__(GRID_THREADS) k_prolong_smooth0(Dev d, MGState m) {
+    pdl_entry();
+    __shared__ float s_cx[GRID_THREADS / 32][216];
+    prolong_smooth0<false>(d, m, 1.0f / coarse_scale(m), s_cx[threadIdx.x >> 5]);
 }
 
 // Levels 1..3 through the active-brick footprints, with the per-solve stencil words; each pass is a
@@ -987,16 +1034,13 @@ __global__ void k_prolong_smooth_fp(Dev d, MGState m, int l) {
 // One warp per brick: the lanes form the fine residuals of the brick's 512 cells in warp-private shared
 // memory, then sum each of the 64 coarse cells' fluid children in child order (x fastest), as the
 // per-coarse-cell loop does.
-__global__ void __launch_bounds__(GRID_THREADS) k_restrict0(Dev d, MGState m) {
-    pdl_entry();
-    constexpr int WARPS = GRID_THREADS / 32;
-    __shared__ float s_res[WARPS][BRICK_CELLS];
-    __shared__ uint8_t s_fluid[WARPS][BRICK_CELLS];
+// res, fluid: the warp's 512 floats and bytes of shared memory; vs: the coarse levels' scale.
+template <bool CL>
+__device__ __forceinline__ void restrict0(const Dev& d, const MGState& m, float vs, float* res, uint8_t* fluid) {
     const MGLevel C = m.lv[1];
-    const float vs = coarse_scale(m);
     const uint32_t active = d.active_bricks[0];
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
-    for (uint32_t e = blockIdx.x * wpb + warp; e < active; e += gridDim.x * wpb) {
+    const uint32_t lane = threadIdx.x & 31u, wpb = blockDim.x >> 5;
+    for (uint32_t e = pass_warp<CL>(); e < active; e += gridDim.x * wpb) {
         const uint4 s0 = *reinterpret_cast<const uint4*>(m.nbr_slots + 8u * e);
         const uint4 s1 = *reinterpret_cast<const uint4*>(m.nbr_slots + 8u * e + 4u);
         const uint32_t ns[6] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y};
@@ -1012,8 +1056,8 @@ __global__ void __launch_bounds__(GRID_THREADS) k_restrict0(Dev d, MGState m) {
                 float n[6];
                 nbrs6(v.z, x, g.h, j, n);
                 const float diag = comp(v.dg, j) + DIAG_EPSILON;
-                s_fluid[warp][g.l + uint32_t(j)] = (w & W_FLUID) ? 1 : 0;
-                if (w & W_FLUID) s_res[warp][g.l + uint32_t(j)] = comp(v.r, j) - (diag * comp(v.z.c, j) - nb_sum(n, w));
+                fluid[g.l + uint32_t(j)] = (w & W_FLUID) ? 1 : 0;
+                if (w & W_FLUID) res[g.l + uint32_t(j)] = comp(v.r, j) - (diag * comp(v.z.c, j) - nb_sum(n, w));
             }
         }
         __syncwarp();
@@ -1035,7 +1079,7 @@ __global__ void __launch_bounds__(GRID_THREADS) k_restrict0(Dev d, MGState m) {
 #pragma unroll
             for (int o = 0; o < 8; ++o) {
                 const uint32_t fl = uint32_t((2 * cl.x + (o & 1)) + 8 * ((2 * cl.y + ((o >> 1) & 1)) + 8 * (2 * cl.z + ((o >> 2) & 1))));
-                if (s_fluid[warp][fl]) sum = sum + s_res[warp][fl];
+                if (fluid[fl]) sum = sum + res[fl];
             }
             const float bb = (m.restrict_scale * sum) * vs;
             lv_st(C.b, ci, C.prec, bb);
@@ -1043,6 +1087,13 @@ __global__ void __launch_bounds__(GRID_THREADS) k_restrict0(Dev d, MGState m) {
         }
         __syncwarp();
     }
+}
+__global__ void __launch_bounds__(GRID_THREADS) k_restrict0(Dev d, MGState m) {
+    pdl_entry();
+    constexpr int WARPS = GRID_THREADS / 32;
+    __shared__ float s_res[WARPS][BRICK_CELLS];
+    __shared__ uint8_t s_fluid[WARPS][BRICK_CELLS];
+    restrict0<false>(d, m, coarse_scale(m), s_res[threadIdx.x >> 5], s_fluid[threadIdx.x >> 5]);
 }
 
 __device__ __forceinline__ float* dir_buf(const MGState& m, uint32_t parity) { return parity ? m.dvec2 : m.dvec; }
@@ -1580,9 +1631,7 @@ __global__ void __launch_bounds__(ST_WARPS * 32) k_update_pr_st(Dev d, MGState m
 // lists), runs the descent, the coarse solve and the ascent there -- every sweep visits only the fluid
 // cells of its colour -- and writes level tail's x back. On entry level `tail` holds b and the
 // red-initialised x from the restriction that produced it.
-__global__ void __launch_bounds__(1024) k_tail_lists(MGState m, int tail) {
-    pdl_entry();
-    __shared__ uint32_t s_warp[33];
+__device__ __forceinline__ void tail_lists(const MGState& m, int tail, uint32_t* s_warp) {  // s_warp: 33 words
     uint32_t off = 0;
     for (int l = tail; l < m.num_levels; ++l) {
         const MGLevel L = m.lv[l];
@@ -1599,7 +1648,7 @@ __global__ void __launch_bounds__(1024) k_tail_lists(MGState m, int tail) {
                 if (lane == 0) s_warp[warp] = __popc(bal);
                 __syncthreads();
                 if (warp == 0) {
-                    const uint32_t v = s_warp[lane];
+                    const uint32_t v = uint32_t(lane) < blockDim.x / 32u ? s_warp[lane] : 0u;
                     uint32_t x = v;
 #pragma unroll
                     for (int o = 1; o < 32; o <<= 1) {
@@ -1639,6 +1688,12 @@ __global__ void __launch_bounds__(1024) k_tail_lists(MGState m, int tail) {
     }
 }
 
+__global__ void __launch_bounds__(1024) k_tail_lists(MGState m, int tail) {
+    pdl_entry();
+    __shared__ uint32_t s_warp[33];
+    tail_lists(m, tail, s_warp);
+}
+
 struct SLevel {
     int3 dim;
     uint32_t cells, dx, dxy;
@@ -1660,30 +1715,48 @@ __device__ __forceinline__ void s_sweep(const SLevel L, uint32_t colour) {
     }
     __syncthreads();
 }
-// The coarsest level's red-black iterations on the first 4 warps, synchronised by a 128-thread named
-// barrier (the level has at most 512 cells, so 128 threads visit each colour in a few rounds).
+// The coarsest level's red-black iterations. It usually has at most 512 cells: thread t holds red cell t and black cell
+// t with their words, right-hand sides and diagonals in registers over all iterations, and a colour costs its
+// neighbours' loads, one division and one barrier of just the warps that hold a cell (a single warp needs none). A level
+// with more cells of a colour than the CTA has threads (grids beyond 2^9 cells an axis) sweeps its lists.
 __device__ __forceinline__ void s_coarse_solve(const SLevel L, int iterations) {
-    if (threadIdx.x < 128u) {
+    const uint32_t threads = (max(max(L.nred, L.nblack), 1u) + 31u) & ~31u;
+    if (threads > blockDim.x) {
+        for (int it = 0; it < iterations; ++it) {
+            s_sweep(L, 0u);
+            s_sweep(L, 1u);
+        }
+        return;
+    }
+    if (threadIdx.x < threads) {
+        uint32_t idx[2], w[2];
+        float b[2], diag[2];
+#pragma unroll
+        for (uint32_t colour = 0; colour < 2u; ++colour) {
+            const bool mine = threadIdx.x < (colour == 0u ? L.nred : L.nblack);
+            idx[colour] = mine ? L.list[threadIdx.x + (colour == 0u ? 0u : L.nred)] : 0xFFFFFFFFu;
+            const uint32_t i = mine ? idx[colour] : 0u;
+            w[colour] = L.word[i];
+            b[colour] = L.b[i];
+            diag[colour] = L.diag[i];
+        }
         for (int it = 0; it < iterations; ++it) {
 #pragma unroll
             for (uint32_t colour = 0; colour < 2u; ++colour) {
-                const uint32_t n = colour == 0u ? L.nred : L.nblack;
-                const uint32_t* list = L.list + (colour == 0u ? 0u : L.nred);
-                for (uint32_t j = threadIdx.x; j < n; j += 128u) {
-                    const uint32_t i = list[j];
-                    const uint32_t w = L.word[i];
-                    L.x[i] = q_prec((L.b[i] + word_sum(L.x, w, i, L.dx, L.dxy)) / L.diag[i], L.prec);
-                }
-                asm volatile("bar.sync 1, 128;" ::: "memory");
+                if (idx[colour] != 0xFFFFFFFFu)
+                    L.x[idx[colour]] = q_prec((b[colour] + word_sum(L.x, w[colour], idx[colour], L.dx, L.dxy)) / diag[colour], L.prec);
+                if (threads == 32u) __syncwarp();
+                else asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
             }
         }
     }
     __syncthreads();
 }
-// The tail's V-cycle on one CTA of 1024 threads (s_tail: mg_tail_smem bytes of shared memory). CG: level tail's x
+// The tail's V-cycle on one CTA (s_tail: mg_tail_smem bytes of shared memory). CG: level tail's x
 // and b were written earlier in the same kernel by other CTAs of the cluster, so they are read through L2.
+// image: also load the solve's static part (false when an earlier call of the same kernel left it there).
 template <bool CG>
-__device__ __forceinline__ void vcycle_tail_body(const MGState& m, int tail, int iterations, unsigned char* s_tail) {
+__device__ __forceinline__ void vcycle_tail_body(const MGState& m, int tail, int iterations, unsigned char* s_tail, bool image = true) {
     const int nl = m.num_levels;
     SLevel S[SLOSH_MAX_MG_LEVELS];
     uint32_t total = 0;
@@ -1708,16 +1781,16 @@ __device__ __forceinline__ void vcycle_tail_body(const MGState& m, int tail, int
     // colour lists of all tail levels) from the image k_tail_lists built for this solve.
     {
         const uint32_t c16 = tail_pad4(m.lv[tail].cells) / 4u;  // 16-byte chunks of one level-tail array
-        const uint32_t n16 = total / 16u;
+        const uint32_t n16 = image ? total / 16u : 2u * c16;
         const uint4* gx = reinterpret_cast<const uint4*>(m.lv[tail].x);
         const uint4* gb = reinterpret_cast<const uint4*>(m.lv[tail].b);
         const uint4* img = reinterpret_cast<const uint4*>(m.tail_image);
         uint4* dst = reinterpret_cast<uint4*>(s_tail);
-        for (uint32_t k0 = 0; k0 < n16; k0 += 8u * 1024u) {
+        for (uint32_t k0 = 0; k0 < n16; k0 += 8u * blockDim.x) {
             uint4 v[8];
 #pragma unroll
             for (int r = 0; r < 8; ++r) {
-                const uint32_t k = k0 + uint32_t(r) * 1024u + threadIdx.x;
+                const uint32_t k = k0 + uint32_t(r) * blockDim.x + threadIdx.x;
                 if (k < n16) {
                     if (k < 2u * c16 && m.lv[tail].prec != SLOSH_PRECISION_FP32) {
                         // 2-byte storage: four elements per 16-byte chunk of shared memory
@@ -1736,7 +1809,7 @@ __device__ __forceinline__ void vcycle_tail_body(const MGState& m, int tail, int
             }
 #pragma unroll
             for (int r = 0; r < 8; ++r) {
-                const uint32_t k = k0 + uint32_t(r) * 1024u + threadIdx.x;
+                const uint32_t k = k0 + uint32_t(r) * blockDim.x + threadIdx.x;
                 if (k < n16) dst[k] = v[r];
             }
         }
@@ -1896,12 +1969,9 @@ __global__ void __launch_bounds__(1024) k_coarse_solve0(Dev d, MGState m, int it
 // the previous direction from one buffer and writes the new one to the other, and forms each fluid
 // neighbour's new direction z_n + beta d_n itself (bit-identical to what that neighbour writes).
 
-__global__ void __launch_bounds__(GRID_THREADS, 3) k_apply_a(Dev d, MGState m) {
-    pdl_entry();
-    const uint32_t it = m.ctl[0];
+template <bool CL, class Store>
+__device__ __forceinline__ void apply_a(const Dev& d, const MGState& m, uint32_t it, float beta, Store store, uint32_t first_partial = 0u) {
     const bool first = it == 0u;
-    // flexible PCG: beta = (rho_k - r_k.z_{k-1}) / rho_{k-1}, the numerator formed in FP64
-    const float beta = first ? 0.0f : ratio_f(m.flexible ? m.scalars[0] - m.scalars[9] : m.scalars[0], m.scalars[3]);
     const float* dold = dir_buf(m, it & 1u);
     float* dnew = dir_buf(m, (it + 1u) & 1u);
     struct V {
@@ -1909,7 +1979,7 @@ __global__ void __launch_bounds__(GRID_THREADS, 3) k_apply_a(Dev d, MGState m) {
         float4 dg;
         uint32_t w;
     };
-    w4_pass<1, 1>(d, m, 2,
+    w4_pass<1, 1, CL>(d, m, 2,
         [&](const Geo& g, const uint32_t* ns) {
             V v;
             v.z = load_q6(m.z, g, ns);
@@ -1943,21 +2013,29 @@ __global__ void __launch_bounds__(GRID_THREADS, 3) k_apply_a(Dev d, MGState m) {
             st4(dnew + g.i, dn);
             st4(m.q + g.i, q);
         },
-        [&](double dq, double) { m.scalars[2] = dq; });
+        store, first_partial);
+}
+// flexible PCG: beta = (rho_k - r_k.z_{k-1}) / rho_{k-1}, the numerator formed in FP64
+__device__ __forceinline__ float pcg_beta(bool first, bool flexible, double rho, double rz, double rho_prev) {
+    return first ? 0.0f : ratio_f(flexible ? rho - rz : rho, rho_prev);
+}
+__global__ void __launch_bounds__(GRID_THREADS, 3) k_apply_a(Dev d, MGState m) {
+    pdl_entry();
+    const uint32_t it = m.ctl[0];
+    const float beta = pcg_beta(it == 0u, m.flexible != 0u, m.scalars[0], m.scalars[9], m.scalars[3]);
+    apply_a<false>(d, m, it, beta, [&](double dq, double) { m.scalars[2] = dq; });
 }
 
 // ---- PCGUpdatePRCS: p += alpha d, r -= alpha q, red pre-smooth; ||r||^2 and the loop decision -------------
 // FLEX (flexible PCG) also reduces r_{k+1}.z_k with the z of the finished V-cycle, before it is overwritten.
-template <bool FLEX>
-__global__ void __launch_bounds__(GRID_THREADS, 3) k_update_pr(Dev d, MGState m, float* __restrict__ p, unsigned long long handle) {
-    pdl_entry();
-    const float alpha = ratio_f(m.scalars[0], m.scalars[2]);
-    const float* dcur = dir_buf(m, (m.ctl[0] + 1u) & 1u);
+template <bool FLEX, bool CL, class Store>
+__device__ __forceinline__ void update_pr(const Dev& d, const MGState& m, float* p, uint32_t it, float alpha, Store store) {
+    const float* dcur = dir_buf(m, (it + 1u) & 1u);
     struct V {
         float4 p, d, r, q, dg, z;
         uint32_t w;
     };
-    w4_pass<FLEX ? 2 : 1, 2>(d, m, 3,
+    w4_pass<FLEX ? 2 : 1, 2, CL>(d, m, 3,
         [&](const Geo& g, const uint32_t*) {
             V v;
             v.p = ld4(p + g.i);
@@ -1989,6 +2067,12 @@ __global__ void __launch_bounds__(GRID_THREADS, 3) k_update_pr(Dev d, MGState m,
             st4(m.r + g.i, ro);
             st4(m.z + g.i, zo);
         },
+        store);
+}
+template <bool FLEX>
+__global__ void __launch_bounds__(GRID_THREADS, 3) k_update_pr(Dev d, MGState m, float* __restrict__ p, unsigned long long handle) {
+    pdl_entry();
+    update_pr<FLEX, false>(d, m, p, m.ctl[0], ratio_f(m.scalars[0], m.scalars[2]),
         [&](double rr, double rz) {
             m.scalars[5] = rr;
             if (FLEX) m.scalars[9] = rz;
@@ -2046,6 +2130,178 @@ __global__ void __launch_bounds__(GRID_THREADS) k_true_residual(Dev d, MGState m
         [&](double num, double den) { m.scalars[6] = num; m.scalars[7] = den; });
 }
 
+// ---- a whole solve in one thread-block cluster ---------------------------------------------------------------
+// A small tank's passes take 3-9 us each as launches (a kernel boundary, the dependent loads that start every pass, the
+// last CTA's reduction), not bandwidth: 11 passes an iteration at 64x64x48. Here one cluster of up to 16 CTAs runs the
+// solve's setup and all of its iterations, every pass being the same per-brick or per-cell body as the launched kernels
+// followed by a cluster barrier (release / acquire). A dot product's brick partials are reduced by every CTA for itself
+// after the barrier, in the canonical order, so all CTAs take the same alpha, beta and stopping decision and the results
+// are bit for bit those of the launched form. Nothing waits on another kernel and the cluster's CTAs are scheduled
+// together, so solves of many tanks run side by side on their own streams; as graphs with a conditional loop they ran
+// almost one after another.
+// Used while the tank had at most CL_MAX_BRICKS active bricks in its last frame: 24 tanks of 70-288 active bricks, two
+// substeps a frame, 36.2 -> 15.9 ms stepped together; one tank of 150 active bricks 1.05 -> 0.96 ms a frame. Beyond that the
+// 16 SMs' loads take longer than launches over all of them.
+constexpr uint32_t CL_MAX_BRICKS = 512;
+constexpr int CL_THREADS = 768;  // 85 registers: the level-0 passes need about 80
+constexpr int CL_WARPS = CL_THREADS / 32;
+constexpr size_t CL_SCRATCH = size_t(CL_WARPS) * (BRICK_CELLS * 5u);  // per warp: 512 floats and 512 bytes (restrict0)
+
+// The canonical reduction (final_reduce) by every CTA; all threads get the sum. Groups of 32 lanes that hold no partial
+// are left out: they would add 0.0.
+__device__ __forceinline__ double cl_reduce(const double* partials, uint32_t n, double* s_w32) {
+    const uint32_t lane = threadIdx.x & 31u, groups = min(32u, max(1u, (n + 31u) / 32u));
+    __syncthreads();  // the previous sum has been read
+    for (uint32_t g = threadIdx.x >> 5; g < groups; g += CL_WARPS) {
+        double v = 0.0;
+        for (uint32_t e = g * 32u + lane; e < n; e += 1024u) v = v + partials[e];
+        v = warp_fold(v);
+        if (lane == 0) s_w32[g] = v;
+    }
+    __syncthreads();
+    double total = s_w32[0];
+    for (uint32_t g = 1; g < groups; ++g) total = total + s_w32[g];
+    return total;
+}
+struct ClSolve {
+    float* p;
+    const float* div;
+    uint32_t limit, tol_mode;
+    double tol;
+    int coarse, tail;
+    uint32_t setup, tail_bytes;
+};
+template <bool FLEX>
+__global__ void __launch_bounds__(CL_THREADS, 1) k_solve_cluster(Dev d, MGState m, ClSolve a) {
+    extern __shared__ __align__(16) unsigned char s_tail[];
+    __shared__ uint32_t s_warp[33];
+    __shared__ double s_sum[2][32];
+    const uint32_t warp = threadIdx.x >> 5;
+    float* scratch = reinterpret_cast<float*>(s_tail + a.tail_bytes + warp * (BRICK_CELLS * 5u));
+    uint8_t* scratch_b = reinterpret_cast<uint8_t*>(scratch + BRICK_CELLS);
+    const int nl = m.num_levels, tail = a.tail, top = min(3, nl - 1), sweeps = max(m.sweeps, 1);
+    const bool relaxed = m.smooth_weight != 1.0f;
+    const uint32_t active = d.active_bricks[0], cap = d.num_pool_bricks;
+    auto no_store = [](double, double) {};
+    if (a.setup) {
+        for (int l = 1; l <= top; ++l)
+            for (uint32_t i = pass_thread<true>(); i < m.lv[l].cells; i += gridDim.x * blockDim.x) m.lv[l].type[i] = 0u;
+        cluster_barrier();
+        build_types_fp13<true>(d, m, top);
+        cluster_barrier();
+        for (int l = top; l < nl - 1; ++l) {
+            const MGLevel F = m.lv[l], C = m.lv[l + 1];
+            for (uint32_t i = pass_thread<true>(); i < C.cells; i += gridDim.x * blockDim.x) build_type_cell(d, F, C, 0, i, coord3(i, C.dim));
+            cluster_barrier();
+        }
+        level_words_fp13<true>(d, m, top);
+        for (int l = top + 1; l < nl; ++l)
+            for (uint32_t i = pass_thread<true>(); i < m.lv[l].cells; i += gridDim.x * blockDim.x) level_word_cell(m.lv[l], i, coord3(i, m.lv[l].dim));
+        pcg_words<true>(d, m);
+        cluster_barrier();
+        if (blockIdx.x == 0u) {
+            tail_lists(m, tail, s_warp);
+            __syncthreads();
+        }
+    }
+    pcg_init<true>(d, m, a.p, a.div, no_store);
+    cluster_barrier();
+    double rr = cl_reduce(m.partials, active, s_sum[0]);
+    const double bb = cl_reduce(m.partials + cap, active, s_sum[1]);
+    double rho = m.scalars[0], rho_prev = 0.0, dq = 0.0, rz = 0.0;
+    uint32_t it = 0u;
+    bool converged = a.tol_mode != 0u && (bb > 0.0 ? sqrt(rr / bb) : 0.0) <= a.tol;
+    bool run = a.limit > 0u && !converged, image = true;
+    while (run) {
+        const float vs = coarse_scale(m, rr), ivs = 1.0f / vs;
+        auto sweep = [&](int l, uint32_t parity) {
+            const MGLevel L = m.lv[l];
+            const uint32_t want = parity == 0u ? CW_RED : 0u;
+            if (l <= 2) for_footprint_colour<true>(d, L, l, parity, [&](uint32_t i, int3) { smooth_fp_cell(L, i, want); });
+            else for_footprint<true>(d, L, l, [&](uint32_t i, int3) { smooth_fp_cell(L, i, want); });
+            cluster_barrier();
+        };
+        smooth0_black<true>(d, m);
+        cluster_barrier();
+        for (int k = 1; k < sweeps; ++k) {
+            smooth0_red<false, false, true>(d, m, ivs);
+            cluster_barrier();
+            smooth0_black<true>(d, m);
+            cluster_barrier();
+        }
+        for (int l = 0; l < tail; ++l) {
+            if (l == 0) {
+                restrict0<true>(d, m, vs, scratch, scratch_b);
+            } else {
+                const MGLevel F = m.lv[l], C = m.lv[l + 1];
+                for_footprint<true>(d, C, l + 1, [&](uint32_t ci, int3 c) { restrict_fp_cell(F, C, ci, c, m.restrict_scale); });
+            }
+            cluster_barrier();
+            if (l + 1 < tail) {
+                sweep(l + 1, 1u);
+                for (int k = 1; k < sweeps; ++k) {
+                    sweep(l + 1, 0u);
+                    sweep(l + 1, 1u);
+                }
+            }
+        }
+        if (blockIdx.x == 0u) vcycle_tail_body<false>(m, tail, a.coarse, s_tail, image);
+        image = false;
+        cluster_barrier();
+        for (int l = tail - 1; l >= 1; --l) {
+            const MGLevel F = m.lv[l], C = m.lv[l + 1];
+            if (l <= 2) for_footprint_colour<true>(d, F, l, 1u, [&](uint32_t i, int3 c) { prolong_smooth_fp_cell(F, C, i, c); });
+            else for_footprint<true>(d, F, l, [&](uint32_t i, int3 c) { prolong_smooth_fp_cell(F, C, i, c); });
+            cluster_barrier();
+            for (int k = 1; k < sweeps; ++k) {
+                sweep(l, 0u);
+                sweep(l, 1u);
+            }
+            sweep(l, 0u);
+        }
+        prolong_smooth0<true>(d, m, ivs, scratch);
+        cluster_barrier();
+        for (int k = 1; k < sweeps; ++k) {
+            if (k == 1 && relaxed) smooth0_red<false, true, true>(d, m, ivs);
+            else smooth0_red<false, false, true>(d, m, ivs);
+            cluster_barrier();
+            smooth0_black<true>(d, m);
+            cluster_barrier();
+        }
+        if (sweeps == 1 && relaxed) smooth0_red<true, true, true>(d, m, ivs);
+        else smooth0_red<true, false, true>(d, m, ivs);
+        cluster_barrier();
+        rho_prev = rho;
+        rho = cl_reduce(m.partials, active, s_sum[0]);
+        // into the other half of the partials: a slower CTA may still be reading rho's
+        apply_a<true>(d, m, it, pcg_beta(it == 0u, FLEX, rho, rz, rho_prev), no_store, cap);
+        cluster_barrier();
+        dq = cl_reduce(m.partials + cap, active, s_sum[1]);
+        if (FLEX) cluster_barrier();  // UpdatePR writes both halves
+        update_pr<FLEX, true>(d, m, a.p, it, ratio_f(rho, dq), no_store);
+        cluster_barrier();
+        rr = cl_reduce(m.partials, active, s_sum[0]);
+        if (FLEX) rz = cl_reduce(m.partials + cap, active, s_sum[1]);
+        ++it;
+        converged = a.tol_mode != 0u && (bb > 0.0 ? sqrt(rr / bb) : 0.0) <= a.tol;
+        run = it < a.limit && !converged;
+    }
+    if (blockIdx.x == 0u && threadIdx.x == 0u) {
+        m.ctl[0] = it;
+        m.ctl[1] = a.limit;
+        m.ctl[2] = a.tol_mode;
+        m.ctl[3] = 1u;
+        if (it > 0u && a.tol_mode != 0u && !converged) m.ctl[4] = 1u;  // stopped at the limit: sticky for the frame
+        m.scalars[0] = rho;
+        m.scalars[2] = dq;
+        m.scalars[3] = rho_prev;
+        m.scalars[4] = bb;
+        m.scalars[5] = rr;
+        m.scalars[8] = a.tol;
+        if (FLEX) m.scalars[9] = rz;
+    }
+}
+
 inline int blocks_for(uint32_t n, int threads) { return int((n + uint32_t(threads) - 1u) / uint32_t(threads)); }
 
 // Level-0 passes straight from global memory (default) or from shared-memory stages filled by bulk copies
@@ -2082,6 +2338,22 @@ int st_grid(K kernel, size_t smem, const Dev& d, const Shape& sh) {
     } while (0)
 #define ST_LAUNCH(kernel, NF, NB, d, m, sh, s) ST_LAUNCH_ARGS(kernel, NF, NB, d, sh, s, d, m)
 inline int st_grid_cap(const Dev& d) { return std::max(1, int((d.num_pool_bricks + uint32_t(ST_WARPS) - 1u) / uint32_t(ST_WARPS))); }
+
+constexpr int CL_MAX_SMEM = 200 * 1024;  // the same for every context: a tail is at most 85 KB
+size_t cl_tail_bytes(const MGState& m) { return (mg_tail_smem(m) + 15u) & ~size_t(15); }
+size_t cl_smem(const MGState& m) { return cl_tail_bytes(m) + CL_SCRATCH; }
+void cl_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, int ctas, size_t smem, cudaStream_t s) {
+    cfg.gridDim = dim3(unsigned(ctas));
+    cfg.blockDim = dim3(CL_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = unsigned(ctas);
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+}
 
 }  // namespace
 
@@ -2134,6 +2406,40 @@ int mid_level(const MGState& m, int tail) {
         checked_smem = smem;
     }
     return ok ? from : 0;
+}
+
+// CTAs of the cluster solve's cluster for this hierarchy on the current device: 16, or 8 where no cluster of 16 can be
+// placed, or 0 (a single level, an alternative form asked for by the environment, no room).
+int mg_solve_cluster(const MGState& m) {
+    if (m.num_levels < 2 || mg_staged() || mid_level(m, mg_tail_level(m)) > 0) return 0;
+    const size_t smem = cl_smem(m);
+    if (smem > size_t(CL_MAX_SMEM)) return 0;
+    for (int ctas : {16, 8}) {
+        bool ok = true;
+        for (int flex = 0; flex < 2 && ok; ++flex) {
+            auto kernel = flex ? k_solve_cluster<true> : k_solve_cluster<false>;
+            cudaLaunchConfig_t cfg = {};
+            cudaLaunchAttribute attr[1];
+            cl_config(cfg, attr, ctas, smem, nullptr);
+            int clusters = 0;
+            ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                 cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CL_MAX_SMEM) == cudaSuccess &&
+                 cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters > 0;
+        }
+        cudaGetLastError();
+        if (ok) return ctas;
+    }
+    return 0;
+}
+uint32_t mg_solve_cluster_bricks() { return CL_MAX_BRICKS; }
+int launch_solve_cluster(const Dev& d, const MGState& m, int ctas, float* p, const float* div, uint32_t limit, bool tol_mode, double tol,
+                         int coarse, bool setup, cudaStream_t s) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    cl_config(cfg, attr, ctas, cl_smem(m), s);
+    const ClSolve a{p, div, limit, tol_mode ? 1u : 0u, tol, coarse, mg_tail_level(m), setup ? 1u : 0u, uint32_t(cl_tail_bytes(m))};
+    cudaLaunchKernelEx(&cfg, m.flexible ? k_solve_cluster<true> : k_solve_cluster<false>, d, m, a);
+    return 1;
 }
 
 int launch_mg_setup(const MGState& m, uint32_t limit, bool tol_mode, double tol, cudaStream_t s) {

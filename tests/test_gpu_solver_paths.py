@@ -32,3 +32,19 @@ def test_rbgs_matches_oracle(slosh, oracle_mod, grid, iterations):
     rg, ro = g.results(), o.results()
     # FP64 sums of the same FP32 terms in two orders
     assert rg.last_solve_true_rel_residual == pytest.approx(ro.last_solve_true_rel_residual, rel=1e-6)
+
+
+# The cluster form of the solve (few active bricks) and the launched form against the oracle: one and two tail levels,
+# levels between level 0 and the tail, fixed counts and a tolerance, every preconditioner option, each storage precision.
+@pytest.mark.parametrize("grid", [(16, 16, 16), (21, 17, 30), (64, 40, 33), (96, 72, 50)])
+@pytest.mark.parametrize("settings", [
+    dict(tolerance=0.0, pcg_iterations=3),
+    dict(tolerance=1e-6, mg_smoothing_sweeps=2, mg_correction_scale=1.9, mg_coarse_iterations=4, mg_smoother_weight=1.15),
+    dict(tolerance=1e-5, precision_mode=A.PRECISION_BF16_STORAGE, pcg_flexible=1, mg_smoothing_sweeps=3),
+    dict(tolerance=1e-5, precision_mode=A.PRECISION_FP16_STORAGE, pcg_flexible=1, mg_smoother_weight=1.15),
+    dict(tolerance=1e-12, max_iterations=2),
+])
+def test_mgpcg_forms_match_oracle(slosh, oracle_mod, grid, settings):
+    sc = _scene(slosh, grid, A.SOLVER_MGPCG, **settings)
+    g, o = pair(slosh, oracle_mod, sc)
+    run_frames(g, o, sc, frames=2, tol=None)
