@@ -172,7 +172,7 @@ struct Ctx {
     SortBuffers sortb{};
     P2GGather gather{};  // the per-cell particle index of the gather P2G (allocated only when it is on)
     MGState mg{};
-    int cluster_ctas = 0;          // CTAs of the cluster form of the solve (0: not available for this layout)
+    uint32_t cluster_sizes = 0;    // cluster sizes of the solve's cluster form for this layout (0: not available)
     uint32_t bricks_estimate = 0;  // active bricks of the last frame; the layout's most before the first
 
     // pinned host staging
@@ -458,7 +458,7 @@ struct Ctx {
         total_emitted = 0;
         prev_dt = 0.0f;
         last_max_speed = 0.0f;
-        cluster_ctas = mg_solve_cluster(mg);
+        cluster_sizes = mg_solve_clusters(mg);
         bricks_estimate = num_pool_bricks - 1u;
         shape.num_sms = num_sms;
         shape.brick_ctas = brick_ctas_for(ctas_per_sm);
@@ -716,9 +716,9 @@ struct Ctx {
         const Dev d = dev();
         // few active bricks: the whole solve in one cluster (the form does not change the result, so the last frame's
         // count, which the host has, is enough to choose by)
-        const bool cluster = cluster_ctas > 0 && bricks_estimate <= mg_solve_cluster_bricks();
+        const int cluster = mg_solve_cluster(cluster_sizes, bricks_estimate);
         SolveGraph* G = nullptr;
-        if (use_graphs && !cluster) {
+        if (use_graphs && cluster == 0) {
             try {
                 G = solve_graph(p, div, limit, tol_mode, tolerance, coarse_iterations, slot == 0);
             } catch (const CudaError& e) {
@@ -728,8 +728,8 @@ struct Ctx {
                 destroy_graphs();
             }
         }
-        if (cluster) {
-            const int n = launch_solve_cluster(d, mg, cluster_ctas, p, div, limit, tol_mode, double(tolerance), coarse_iterations, slot == 0, stream);
+        if (cluster > 0) {
+            const int n = launch_solve_cluster(d, mg, cluster, p, div, limit, tol_mode, double(tolerance), coarse_iterations, slot == 0, stream);
             frame_solves.push_back({n, 0, slot});
         } else if (G) {
             CK(cudaGraphLaunch(G->exec, stream));

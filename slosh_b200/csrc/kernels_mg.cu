@@ -109,10 +109,10 @@ __device__ __forceinline__ void stencil0(const Dev& d, const float* buf, uint32_
 }
 
 // Shared-memory layout of the tail levels (byte offsets; every array padded to 4 cells, so each starts
-// on 16 bytes): per level x, b, diag (f32), word (u16), colour list (u32; red then black). Level `tail`'s
+// on 16 bytes): per level x, b (f32), word (u16), colour list (u32; red then black). Level `tail`'s
 // x and b come first. The same layout is used for the per-solve image in global memory.
 struct TailOffsets {
-    uint32_t x, b, diag, word, list;
+    uint32_t x, b, word, list;
 };
 __host__ __device__ __forceinline__ uint32_t tail_pad4(uint32_t cells) { return (cells + 3u) & ~3u; }
 __host__ __device__ __forceinline__ TailOffsets tail_offsets(const MGState& m, int tail, int level, uint32_t* total) {
@@ -123,7 +123,6 @@ __host__ __device__ __forceinline__ TailOffsets tail_offsets(const MGState& m, i
         TailOffsets t;
         t.x = off; off += c4 * 4u;
         t.b = off; off += c4 * 4u;
-        t.diag = off; off += c4 * 4u;
         t.word = off; off += (c4 * 2u + 15u) & ~15u;
         t.list = off; off += c4 * 4u;
         if (l == level) o = t;
@@ -471,6 +470,17 @@ __global__ void __launch_bounds__(GRID_THREADS) k_rbgs(Dev d, MGState m, float* 
     }
 }
 
+// a / d correctly rounded, rc = the correctly rounded 1 / d (Markstein's theorem, IBM J. Res. Dev. 34 (1), 1990: a
+// faithful quotient corrected once by its exact remainder times rc is the rounded quotient; the first correction makes
+// the product faithful). Five dependent operations where the division takes about 200 cycles. The remainders are exact
+// only away from the ends of the exponent range: outside [1e-25, 1e25] the division itself.
+__device__ __forceinline__ float div_by(float a, float d, float rc) {
+    const float m = fabsf(a);
+    if (!(m >= 1e-25f && m <= 1e25f)) return a == 0.0f ? a * rc : a / d;
+    float q = a * rc;
+    q = __fmaf_rn(__fmaf_rn(-q, d, a), rc, q);
+    return __fmaf_rn(__fmaf_rn(-q, d, a), rc, q);
+}
 struct Nb6 {
     uint32_t w;
     float c0, c1, c2;
@@ -1627,7 +1637,7 @@ __global__ void __launch_bounds__(ST_WARPS * 32) k_update_pr_st(Dev d, MGState m
 
 // ---- the small coarse levels in one CTA: levels tail..nl-1 of the V-cycle --------------------------------
 // Once per solve, k_tail_lists stores each tail level's fluid cells by colour. Each V-cycle,
-// k_vcycle_tail copies the tail levels into shared memory (word, diagonal, x, b per cell; the colour
+// k_vcycle_tail copies the tail levels into shared memory (word, x, b per cell; the colour
 // lists), runs the descent, the coarse solve and the ascent there -- every sweep visits only the fluid
 // cells of its colour -- and writes level tail's x back. On entry level `tail` holds b and the
 // red-initialised x from the restriction that produced it.
@@ -1670,18 +1680,15 @@ __device__ __forceinline__ void tail_lists(const MGState& m, int tail, uint32_t*
             off += base;
         }
     }
-    // The static part of the tail's shared-memory image for this solve: diagonals, words, colour lists.
+    // The static part of the tail's shared-memory image for this solve: words, colour lists.
     __syncthreads();
     for (int l = tail; l < m.num_levels; ++l) {
         const MGLevel L = m.lv[l];
         const TailOffsets o = tail_offsets(m, tail, l, nullptr);
-        float* diag = reinterpret_cast<float*>(m.tail_image + o.diag);
         uint16_t* word = reinterpret_cast<uint16_t*>(m.tail_image + o.word);
         uint32_t* list = reinterpret_cast<uint32_t*>(m.tail_image + o.list);
         for (uint32_t i = threadIdx.x; i < L.cells; i += blockDim.x) {
-            const uint32_t w = L.word[i];
-            word[i] = uint16_t(w);
-            diag[i] = word_diag(w);
+            word[i] = L.word[i];
         }
         const uint32_t first = m.tail_meta[4 * l], n = m.tail_meta[4 * l + 1] + m.tail_meta[4 * l + 3];
         for (uint32_t j = threadIdx.x; j < n; j += blockDim.x) list[j] = m.tail_list[first + j];
@@ -1698,20 +1705,22 @@ struct SLevel {
     int3 dim;
     uint32_t cells, dx, dxy;
     uint16_t* word;
-    float* diag;
+    const float* dt;       // by count of non-solid neighbours: the diagonal (0-6), its reciprocal (8-14)
     float* x;
     float* b;
     const uint32_t* list;  // red cells then black cells
     uint32_t nred, nblack;
     uint32_t prec;         // storage precision: stores round to it (the values stay FP32 in shared memory)
 };
+__device__ __forceinline__ uint32_t word_nonsolid(uint32_t w) { return uint32_t(__popc((w >> CW_NONSOLID_SHIFT) & 63u)); }
 __device__ __forceinline__ void s_sweep(const SLevel L, uint32_t colour) {
     const uint32_t n = colour == 0u ? L.nred : L.nblack;
     const uint32_t* list = L.list + (colour == 0u ? 0u : L.nred);
     for (uint32_t j = threadIdx.x; j < n; j += blockDim.x) {
         const uint32_t i = list[j];
         const uint32_t w = L.word[i];
-        L.x[i] = q_prec((L.b[i] + word_sum(L.x, w, i, L.dx, L.dxy)) / L.diag[i], L.prec);
+        const uint32_t c = word_nonsolid(w);
+        L.x[i] = q_prec(div_by(L.b[i] + word_sum(L.x, w, i, L.dx, L.dxy), L.dt[c], L.dt[8u + c]), L.prec);
     }
     __syncthreads();
 }
@@ -1729,8 +1738,8 @@ __device__ __forceinline__ void s_coarse_solve(const SLevel L, int iterations) {
         return;
     }
     if (threadIdx.x < threads) {
-        uint32_t idx[2], w[2];
-        float b[2], diag[2];
+        uint32_t idx[2], w[2], off[2][6];
+        float b[2], diag[2], rc[2];
 #pragma unroll
         for (uint32_t colour = 0; colour < 2u; ++colour) {
             const bool mine = threadIdx.x < (colour == 0u ? L.nred : L.nblack);
@@ -1738,13 +1747,24 @@ __device__ __forceinline__ void s_coarse_solve(const SLevel L, int iterations) {
             const uint32_t i = mine ? idx[colour] : 0u;
             w[colour] = L.word[i];
             b[colour] = L.b[i];
-            diag[colour] = L.diag[i];
+            diag[colour] = L.dt[word_nonsolid(w[colour])];
+            rc[colour] = L.dt[8u + word_nonsolid(w[colour])];
+            const uint32_t nb[6] = {i - 1u, i + 1u, i - L.dx, i + L.dx, i - L.dxy, i + L.dxy};
+#pragma unroll
+            for (int n = 0; n < 6; ++n) off[colour][n] = ((w[colour] >> n) & 1u) ? nb[n] : i;  // all six load, the fluid ones count
         }
         for (int it = 0; it < iterations; ++it) {
 #pragma unroll
             for (uint32_t colour = 0; colour < 2u; ++colour) {
-                if (idx[colour] != 0xFFFFFFFFu)
-                    L.x[idx[colour]] = q_prec((b[colour] + word_sum(L.x, w[colour], idx[colour], L.dx, L.dxy)) / diag[colour], L.prec);
+                if (idx[colour] != 0xFFFFFFFFu) {
+                    float v[6], sum = 0.0f;
+#pragma unroll
+                    for (int n = 0; n < 6; ++n) v[n] = L.x[off[colour][n]];
+#pragma unroll
+                    for (int n = 0; n < 6; ++n)
+                        if ((w[colour] >> n) & 1u) sum = sum + v[n];
+                    L.x[idx[colour]] = q_prec(div_by(b[colour] + sum, diag[colour], rc[colour]), L.prec);
+                }
                 if (threads == 32u) __syncwarp();
                 else asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
             }
@@ -1752,32 +1772,108 @@ __device__ __forceinline__ void s_coarse_solve(const SLevel L, int iterations) {
     }
     __syncthreads();
 }
+// Descriptors of the tail's levels and the diagonals' table (16 floats) in shared memory, by the CTA's first threads; read
+// after a barrier. A coarse diagonal has seven values: DiagEpsilon and one per non-solid neighbour (word_diag).
+__device__ __forceinline__ void tail_levels(const MGState& m, int tail, unsigned char* s_tail, SLevel* S, float* dt) {
+    if (threadIdx.x < 7u) {
+        dt[threadIdx.x] = word_diag(((1u << threadIdx.x) - 1u) << CW_NONSOLID_SHIFT);
+        dt[8u + threadIdx.x] = 1.0f / dt[threadIdx.x];
+    }
+    const int l = tail + int(threadIdx.x);
+    if (l >= m.num_levels) return;
+    const MGLevel G = m.lv[l];
+    const TailOffsets o = tail_offsets(m, tail, l, nullptr);
+    SLevel L;
+    L.dim = G.dim;
+    L.cells = G.cells;
+    L.dx = uint32_t(G.dim.x);
+    L.dxy = uint32_t(G.dim.x * G.dim.y);
+    L.x = reinterpret_cast<float*>(s_tail + o.x);
+    L.b = reinterpret_cast<float*>(s_tail + o.b);
+    L.dt = dt;
+    L.word = reinterpret_cast<uint16_t*>(s_tail + o.word);
+    L.list = reinterpret_cast<const uint32_t*>(s_tail + o.list);
+    L.nred = m.tail_meta[4 * l + 1];
+    L.nblack = m.tail_meta[4 * l + 3];
+    L.prec = G.prec;
+    S[l] = L;
+}
+// The V-cycle's levels tail..nl-1 in shared memory, level tail's x and b and the static image in place.
+__device__ __forceinline__ void vcycle_tail_levels(const MGState& m, int tail, int iterations, const SLevel* S) {
+    const int nl = m.num_levels;
+    // pre-smoothing of a level: its black half (the red half is the restriction's initialisation), then
+    // m.sweeps - 1 more red-black pairs
+    auto pre_smooth = [&](const SLevel& L) {
+        s_sweep(L, 1u);
+        for (int k = 1; k < m.sweeps; ++k) {
+            s_sweep(L, 0u);
+            s_sweep(L, 1u);
+        }
+    };
+    if (tail < nl - 1) pre_smooth(S[tail]);
+    for (int l = tail; l < nl - 1; ++l) {
+        const SLevel F = S[l];
+        const SLevel C = S[l + 1];
+        // eight lanes per coarse cell, one for each child's residual; the first adds the fluid ones in child order
+        const uint32_t o = threadIdx.x & 7u, lead = threadIdx.x & 24u;
+        for (uint32_t j0 = 0; j0 < C.nred + C.nblack; j0 += blockDim.x / 8u) {
+            const uint32_t j = j0 + threadIdx.x / 8u;
+            const uint32_t ci = j < C.nred + C.nblack ? C.list[j] : 0u;
+            const int3 c = coord3(ci, C.dim);
+            const int3 f = make_int3(c.x * 2 + int(o & 1u), c.y * 2 + int((o >> 1) & 1u), c.z * 2 + int(o >> 2));
+            float res = 0.0f;
+            bool fluid = false;
+            if (inside3(f, F.dim)) {
+                const uint32_t fi = lin3(f, F.dim), w = F.word[fi];
+                fluid = (w & CW_FLUID) != 0u;
+                if (fluid) res = F.b[fi] - (F.dt[word_nonsolid(w)] * F.x[fi] - word_sum(F.x, w, fi, F.dx, F.dxy));
+            }
+            const uint32_t fl = __ballot_sync(0xFFFFFFFFu, fluid) >> lead;
+            float sum = 0.0f;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const float v = __shfl_sync(0xFFFFFFFFu, res, int(lead) + k);
+                if ((fl >> k) & 1u) sum = sum + v;
+            }
+            if (o == 0u && j < C.nred + C.nblack) {
+                const float bb = m.restrict_scale * sum;
+                C.b[ci] = q_prec(bb, C.prec);
+                const uint32_t w = C.word[ci], n = word_nonsolid(w);
+                C.x[ci] = q_prec((w & CW_RED) ? div_by(bb, C.dt[n], C.dt[8u + n]) : 0.0f, C.prec);
+            }
+        }
+        __syncthreads();
+        if (l + 1 < nl - 1) pre_smooth(C);
+    }
+    s_coarse_solve(S[nl - 1], iterations);
+    for (int l = nl - 2; l >= tail; --l) {
+        const SLevel F = S[l];
+        const SLevel C = S[l + 1];
+        for (uint32_t j = threadIdx.x; j < F.nred + F.nblack; j += blockDim.x) {
+            const uint32_t i = F.list[j];
+            const int3 c = coord3(i, F.dim);
+            const uint32_t pi = lin3(make_int3(c.x / 2, c.y / 2, c.z / 2), C.dim);
+            if (C.word[pi] & CW_FLUID) F.x[i] = q_prec(F.x[i] + C.x[pi], F.prec);
+        }
+        __syncthreads();
+        for (int k = 0; k < m.sweeps; ++k) {
+            s_sweep(F, 1u);
+            s_sweep(F, 0u);
+        }
+    }
+}
+
 // The tail's V-cycle on one CTA (s_tail: mg_tail_smem bytes of shared memory). CG: level tail's x
 // and b were written earlier in the same kernel by other CTAs of the cluster, so they are read through L2.
 // image: also load the solve's static part (false when an earlier call of the same kernel left it there).
 template <bool CG>
 __device__ __forceinline__ void vcycle_tail_body(const MGState& m, int tail, int iterations, unsigned char* s_tail, bool image = true) {
-    const int nl = m.num_levels;
-    SLevel S[SLOSH_MAX_MG_LEVELS];
+    __shared__ SLevel s_levels[SLOSH_MAX_MG_LEVELS];
+    __shared__ float s_dt[16];
+    tail_levels(m, tail, s_tail, s_levels, s_dt);
     uint32_t total = 0;
-    for (int l = tail; l < nl; ++l) {
-        const MGLevel G = m.lv[l];
-        const TailOffsets o = tail_offsets(m, tail, l, &total);
-        SLevel& L = S[l];
-        L.dim = G.dim;
-        L.cells = G.cells;
-        L.dx = uint32_t(G.dim.x);
-        L.dxy = uint32_t(G.dim.x * G.dim.y);
-        L.x = reinterpret_cast<float*>(s_tail + o.x);
-        L.b = reinterpret_cast<float*>(s_tail + o.b);
-        L.diag = reinterpret_cast<float*>(s_tail + o.diag);
-        L.word = reinterpret_cast<uint16_t*>(s_tail + o.word);
-        L.list = reinterpret_cast<const uint32_t*>(s_tail + o.list);
-        L.nred = m.tail_meta[4 * l + 1];
-        L.nblack = m.tail_meta[4 * l + 3];
-        L.prec = G.prec;
-    }
-    // One round trip: level tail's x and b from the level arrays, everything static (diagonals, words,
+    tail_offsets(m, tail, -1, &total);
+    // One round trip: level tail's x and b from the level arrays, everything static (words,
     // colour lists of all tail levels) from the image k_tail_lists built for this solve.
     {
         const uint32_t c16 = tail_pad4(m.lv[tail].cells) / 4u;  // 16-byte chunks of one level-tail array
@@ -1815,62 +1911,7 @@ __device__ __forceinline__ void vcycle_tail_body(const MGState& m, int tail, int
         }
     }
     __syncthreads();
-    // pre-smoothing of a level: its black half (the red half is the restriction's initialisation), then
-    // m.sweeps - 1 more red-black pairs
-    auto pre_smooth = [&](const SLevel& L) {
-        s_sweep(L, 1u);
-        for (int k = 1; k < m.sweeps; ++k) {
-            s_sweep(L, 0u);
-            s_sweep(L, 1u);
-        }
-    };
-    if (tail < nl - 1) pre_smooth(S[tail]);
-    for (int l = tail; l < nl - 1; ++l) {
-        const SLevel F = S[l];
-        const SLevel C = S[l + 1];
-        for (uint32_t j = threadIdx.x; j < C.nred + C.nblack; j += blockDim.x) {
-            const uint32_t ci = C.list[j];
-            const int3 c = coord3(ci, C.dim);
-            float res[8];
-            uint32_t fl = 0u;
-#pragma unroll
-            for (int o = 0; o < 8; ++o) {
-                res[o] = 0.0f;
-                const int3 f = make_int3(c.x * 2 + (o & 1), c.y * 2 + ((o >> 1) & 1), c.z * 2 + ((o >> 2) & 1));
-                if (!inside3(f, F.dim)) continue;
-                const uint32_t fi = lin3(f, F.dim);
-                const uint32_t w = F.word[fi];
-                if (!(w & CW_FLUID)) continue;
-                fl |= 1u << o;
-                res[o] = F.b[fi] - (F.diag[fi] * F.x[fi] - word_sum(F.x, w, fi, F.dx, F.dxy));
-            }
-            float sum = 0.0f;
-#pragma unroll
-            for (int o = 0; o < 8; ++o)
-                if ((fl >> o) & 1u) sum = sum + res[o];
-            const float bb = m.restrict_scale * sum;
-            C.b[ci] = q_prec(bb, C.prec);
-            C.x[ci] = q_prec((C.word[ci] & CW_RED) ? bb / C.diag[ci] : 0.0f, C.prec);
-        }
-        __syncthreads();
-        if (l + 1 < nl - 1) pre_smooth(C);
-    }
-    s_coarse_solve(S[nl - 1], iterations);
-    for (int l = nl - 2; l >= tail; --l) {
-        const SLevel F = S[l];
-        const SLevel C = S[l + 1];
-        for (uint32_t j = threadIdx.x; j < F.nred + F.nblack; j += blockDim.x) {
-            const uint32_t i = F.list[j];
-            const int3 c = coord3(i, F.dim);
-            const uint32_t pi = lin3(make_int3(c.x / 2, c.y / 2, c.z / 2), C.dim);
-            if (C.word[pi] & CW_FLUID) F.x[i] = q_prec(F.x[i] + C.x[pi], F.prec);
-        }
-        __syncthreads();
-        for (int k = 0; k < m.sweeps; ++k) {
-            s_sweep(F, 1u);
-            s_sweep(F, 0u);
-        }
-    }
+    vcycle_tail_levels(m, tail, iterations, s_levels);
     {
         const uint32_t c16 = tail_pad4(m.lv[tail].cells) / 4u;
         const uint4* src = reinterpret_cast<const uint4*>(s_tail);
@@ -2130,177 +2171,7 @@ __global__ void __launch_bounds__(GRID_THREADS) k_true_residual(Dev d, MGState m
         [&](double num, double den) { m.scalars[6] = num; m.scalars[7] = den; });
 }
 
-// ---- a whole solve in one thread-block cluster ---------------------------------------------------------------
-// A small tank's passes take 3-9 us each as launches (a kernel boundary, the dependent loads that start every pass, the
-// last CTA's reduction), not bandwidth: 11 passes an iteration at 64x64x48. Here one cluster of up to 16 CTAs runs the
-// solve's setup and all of its iterations, every pass being the same per-brick or per-cell body as the launched kernels
-// followed by a cluster barrier (release / acquire). A dot product's brick partials are reduced by every CTA for itself
-// after the barrier, in the canonical order, so all CTAs take the same alpha, beta and stopping decision and the results
-// are bit for bit those of the launched form. Nothing waits on another kernel and the cluster's CTAs are scheduled
-// together, so solves of many tanks run side by side on their own streams; as graphs with a conditional loop they ran
-// almost one after another.
-// Used while the tank had at most CL_MAX_BRICKS active bricks in its last frame: 24 tanks of 70-288 active bricks, two
-// substeps a frame, 36.2 -> 15.9 ms stepped together; one tank of 150 active bricks 1.05 -> 0.96 ms a frame. Beyond that the
-// 16 SMs' loads take longer than launches over all of them.
-constexpr uint32_t CL_MAX_BRICKS = 512;
-constexpr int CL_THREADS = 768;  // 85 registers: the level-0 passes need about 80
-constexpr int CL_WARPS = CL_THREADS / 32;
-constexpr size_t CL_SCRATCH = size_t(CL_WARPS) * (BRICK_CELLS * 5u);  // per warp: 512 floats and 512 bytes (restrict0)
-
-// The canonical reduction (final_reduce) by every CTA; all threads get the sum. Groups of 32 lanes that hold no partial
-// are left out: they would add 0.0.
-__device__ __forceinline__ double cl_reduce(const double* partials, uint32_t n, double* s_w32) {
-    const uint32_t lane = threadIdx.x & 31u, groups = min(32u, max(1u, (n + 31u) / 32u));
-    __syncthreads();  // the previous sum has been read
-    for (uint32_t g = threadIdx.x >> 5; g < groups; g += CL_WARPS) {
-        double v = 0.0;
-        for (uint32_t e = g * 32u + lane; e < n; e += 1024u) v = v + partials[e];
-        v = warp_fold(v);
-        if (lane == 0) s_w32[g] = v;
-    }
-    __syncthreads();
-    double total = s_w32[0];
-    for (uint32_t g = 1; g < groups; ++g) total = total + s_w32[g];
-    return total;
-}
-struct ClSolve {
-    float* p;
-    const float* div;
-    uint32_t limit, tol_mode;
-    double tol;
-    int coarse, tail;
-    uint32_t setup, tail_bytes;
-};
-template <bool FLEX>
-__global__ void __launch_bounds__(CL_THREADS, 1) k_solve_cluster(Dev d, MGState m, ClSolve a) {
-    extern __shared__ __align__(16) unsigned char s_tail[];
-    __shared__ uint32_t s_warp[33];
-    __shared__ double s_sum[2][32];
-    const uint32_t warp = threadIdx.x >> 5;
-    float* scratch = reinterpret_cast<float*>(s_tail + a.tail_bytes + warp * (BRICK_CELLS * 5u));
-    uint8_t* scratch_b = reinterpret_cast<uint8_t*>(scratch + BRICK_CELLS);
-    const int nl = m.num_levels, tail = a.tail, top = min(3, nl - 1), sweeps = max(m.sweeps, 1);
-    const bool relaxed = m.smooth_weight != 1.0f;
-    const uint32_t active = d.active_bricks[0], cap = d.num_pool_bricks;
-    auto no_store = [](double, double) {};
-    if (a.setup) {
-        for (int l = 1; l <= top; ++l)
-            for (uint32_t i = pass_thread<true>(); i < m.lv[l].cells; i += gridDim.x * blockDim.x) m.lv[l].type[i] = 0u;
-        cluster_barrier();
-        build_types_fp13<true>(d, m, top);
-        cluster_barrier();
-        for (int l = top; l < nl - 1; ++l) {
-            const MGLevel F = m.lv[l], C = m.lv[l + 1];
-            for (uint32_t i = pass_thread<true>(); i < C.cells; i += gridDim.x * blockDim.x) build_type_cell(d, F, C, 0, i, coord3(i, C.dim));
-            cluster_barrier();
-        }
-        level_words_fp13<true>(d, m, top);
-        for (int l = top + 1; l < nl; ++l)
-            for (uint32_t i = pass_thread<true>(); i < m.lv[l].cells; i += gridDim.x * blockDim.x) level_word_cell(m.lv[l], i, coord3(i, m.lv[l].dim));
-        pcg_words<true>(d, m);
-        cluster_barrier();
-        if (blockIdx.x == 0u) {
-            tail_lists(m, tail, s_warp);
-            __syncthreads();
-        }
-    }
-    pcg_init<true>(d, m, a.p, a.div, no_store);
-    cluster_barrier();
-    double rr = cl_reduce(m.partials, active, s_sum[0]);
-    const double bb = cl_reduce(m.partials + cap, active, s_sum[1]);
-    double rho = m.scalars[0], rho_prev = 0.0, dq = 0.0, rz = 0.0;
-    uint32_t it = 0u;
-    bool converged = a.tol_mode != 0u && (bb > 0.0 ? sqrt(rr / bb) : 0.0) <= a.tol;
-    bool run = a.limit > 0u && !converged, image = true;
-    while (run) {
-        const float vs = coarse_scale(m, rr), ivs = 1.0f / vs;
-        auto sweep = [&](int l, uint32_t parity) {
-            const MGLevel L = m.lv[l];
-            const uint32_t want = parity == 0u ? CW_RED : 0u;
-            if (l <= 2) for_footprint_colour<true>(d, L, l, parity, [&](uint32_t i, int3) { smooth_fp_cell(L, i, want); });
-            else for_footprint<true>(d, L, l, [&](uint32_t i, int3) { smooth_fp_cell(L, i, want); });
-            cluster_barrier();
-        };
-        smooth0_black<true>(d, m);
-        cluster_barrier();
-        for (int k = 1; k < sweeps; ++k) {
-            smooth0_red<false, false, true>(d, m, ivs);
-            cluster_barrier();
-            smooth0_black<true>(d, m);
-            cluster_barrier();
-        }
-        for (int l = 0; l < tail; ++l) {
-            if (l == 0) {
-                restrict0<true>(d, m, vs, scratch, scratch_b);
-            } else {
-                const MGLevel F = m.lv[l], C = m.lv[l + 1];
-                for_footprint<true>(d, C, l + 1, [&](uint32_t ci, int3 c) { restrict_fp_cell(F, C, ci, c, m.restrict_scale); });
-            }
-            cluster_barrier();
-            if (l + 1 < tail) {
-                sweep(l + 1, 1u);
-                for (int k = 1; k < sweeps; ++k) {
-                    sweep(l + 1, 0u);
-                    sweep(l + 1, 1u);
-                }
-            }
-        }
-        if (blockIdx.x == 0u) vcycle_tail_body<false>(m, tail, a.coarse, s_tail, image);
-        image = false;
-        cluster_barrier();
-        for (int l = tail - 1; l >= 1; --l) {
-            const MGLevel F = m.lv[l], C = m.lv[l + 1];
-            if (l <= 2) for_footprint_colour<true>(d, F, l, 1u, [&](uint32_t i, int3 c) { prolong_smooth_fp_cell(F, C, i, c); });
-            else for_footprint<true>(d, F, l, [&](uint32_t i, int3 c) { prolong_smooth_fp_cell(F, C, i, c); });
-            cluster_barrier();
-            for (int k = 1; k < sweeps; ++k) {
-                sweep(l, 0u);
-                sweep(l, 1u);
-            }
-            sweep(l, 0u);
-        }
-        prolong_smooth0<true>(d, m, ivs, scratch);
-        cluster_barrier();
-        for (int k = 1; k < sweeps; ++k) {
-            if (k == 1 && relaxed) smooth0_red<false, true, true>(d, m, ivs);
-            else smooth0_red<false, false, true>(d, m, ivs);
-            cluster_barrier();
-            smooth0_black<true>(d, m);
-            cluster_barrier();
-        }
-        if (sweeps == 1 && relaxed) smooth0_red<true, true, true>(d, m, ivs);
-        else smooth0_red<true, false, true>(d, m, ivs);
-        cluster_barrier();
-        rho_prev = rho;
-        rho = cl_reduce(m.partials, active, s_sum[0]);
-        // into the other half of the partials: a slower CTA may still be reading rho's
-        apply_a<true>(d, m, it, pcg_beta(it == 0u, FLEX, rho, rz, rho_prev), no_store, cap);
-        cluster_barrier();
-        dq = cl_reduce(m.partials + cap, active, s_sum[1]);
-        if (FLEX) cluster_barrier();  // UpdatePR writes both halves
-        update_pr<FLEX, true>(d, m, a.p, it, ratio_f(rho, dq), no_store);
-        cluster_barrier();
-        rr = cl_reduce(m.partials, active, s_sum[0]);
-        if (FLEX) rz = cl_reduce(m.partials + cap, active, s_sum[1]);
-        ++it;
-        converged = a.tol_mode != 0u && (bb > 0.0 ? sqrt(rr / bb) : 0.0) <= a.tol;
-        run = it < a.limit && !converged;
-    }
-    if (blockIdx.x == 0u && threadIdx.x == 0u) {
-        m.ctl[0] = it;
-        m.ctl[1] = a.limit;
-        m.ctl[2] = a.tol_mode;
-        m.ctl[3] = 1u;
-        if (it > 0u && a.tol_mode != 0u && !converged) m.ctl[4] = 1u;  // stopped at the limit: sticky for the frame
-        m.scalars[0] = rho;
-        m.scalars[2] = dq;
-        m.scalars[3] = rho_prev;
-        m.scalars[4] = bb;
-        m.scalars[5] = rr;
-        m.scalars[8] = a.tol;
-        if (FLEX) m.scalars[9] = rz;
-    }
-}
+#include "mg_cluster.cuh"
 
 inline int blocks_for(uint32_t n, int threads) { return int((n + uint32_t(threads) - 1u) / uint32_t(threads)); }
 
@@ -2339,9 +2210,9 @@ int st_grid(K kernel, size_t smem, const Dev& d, const Shape& sh) {
 #define ST_LAUNCH(kernel, NF, NB, d, m, sh, s) ST_LAUNCH_ARGS(kernel, NF, NB, d, sh, s, d, m)
 inline int st_grid_cap(const Dev& d) { return std::max(1, int((d.num_pool_bricks + uint32_t(ST_WARPS) - 1u) / uint32_t(ST_WARPS))); }
 
-constexpr int CL_MAX_SMEM = 200 * 1024;  // the same for every context: a tail is at most 85 KB
+constexpr int CL_MAX_SMEM = 214 * 1024;  // the same for every context: a tail is at most 65 KB
 size_t cl_tail_bytes(const MGState& m) { return (mg_tail_smem(m) + 15u) & ~size_t(15); }
-size_t cl_smem(const MGState& m) { return cl_tail_bytes(m) + CL_SCRATCH; }
+size_t cl_smem(const MGState& m) { return std::max(cl_tail_bytes(m) + CL_SCRATCH, CL_BLOCKS); }
 void cl_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, int ctas, size_t smem, cudaStream_t s) {
     cfg.gridDim = dim3(unsigned(ctas));
     cfg.blockDim = dim3(CL_THREADS);
@@ -2408,13 +2279,14 @@ int mid_level(const MGState& m, int tail) {
     return ok ? from : 0;
 }
 
-// CTAs of the cluster solve's cluster for this hierarchy on the current device: 16, or 8 where no cluster of 16 can be
-// placed, or 0 (a single level, an alternative form asked for by the environment, no room).
-int mg_solve_cluster(const MGState& m) {
-    if (m.num_levels < 2 || mg_staged() || mid_level(m, mg_tail_level(m)) > 0) return 0;
+// The cluster sizes that the solve of this hierarchy can run with on the current device: bit c for a cluster of c CTAs (4
+// to 16, even). 0: none (a single level, an alternative form asked for by the environment, no room).
+uint32_t mg_solve_clusters(const MGState& m) {
+    if (m.num_levels < 2 || mg_staged() || mid_level(m, mg_tail_level(m)) > 0) return 0u;
     const size_t smem = cl_smem(m);
-    if (smem > size_t(CL_MAX_SMEM)) return 0;
-    for (int ctas : {16, 8}) {
+    if (smem > size_t(CL_MAX_SMEM)) return 0u;
+    uint32_t sizes = 0u;
+    for (int ctas = 4; ctas <= 16; ctas += 2) {
         bool ok = true;
         for (int flex = 0; flex < 2 && ok; ++flex) {
             auto kernel = flex ? k_solve_cluster<true> : k_solve_cluster<false>;
@@ -2427,11 +2299,20 @@ int mg_solve_cluster(const MGState& m) {
                  cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters > 0;
         }
         cudaGetLastError();
-        if (ok) return ctas;
+        if (ok) sizes |= 1u << ctas;
     }
+    return sizes;
+}
+// The cluster for a tank of about `bricks` active bricks: the smallest whose resident form holds them with a sixteenth to
+// spare, so that several tanks' clusters fit the GPU at once (a solve's passes take as long on few SMs as on many while
+// each warp has one brick). 0, the launched form, for tanks that no cluster holds: the streamed form, which takes over
+// when a tank outgrows its cluster within a frame, is slower than launches over the whole GPU (64^3, 240 to 300 active
+// bricks: 1.8 against 1.3 ms a frame).
+int mg_solve_cluster(uint32_t sizes, uint32_t bricks) {
+    for (int ctas = 4; ctas <= 16; ctas += 2)
+        if (((sizes >> ctas) & 1u) && bricks + bricks / 16u <= uint32_t(ctas - 1) * uint32_t(CL_WARPS)) return ctas;
     return 0;
 }
-uint32_t mg_solve_cluster_bricks() { return CL_MAX_BRICKS; }
 int launch_solve_cluster(const Dev& d, const MGState& m, int ctas, float* p, const float* div, uint32_t limit, bool tol_mode, double tol,
                          int coarse, bool setup, cudaStream_t s) {
     cudaLaunchConfig_t cfg = {};
