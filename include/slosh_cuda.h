@@ -364,7 +364,7 @@ SLOSH_API slosh_status slosh_sort_particles(void* ctx);
  * SLOSH_ERR_CAPACITY. The array's address differs per CUDA context; each call looks up the current
  * context's and resolves it on the first call in that context. That first call also loads the library's
  * device code into the context if CUDA has not loaded it yet (lazy module loading is the default), which
- * commits about 7.4 MB of device memory for the scratch, and it is the only call that allocates: make it
+ * commits about 6.3 MB of device memory for the scratch, and it is the only call that allocates: make it
  * at start-up, before any stream capture begins in that context (CUDA_MODULE_LOADING=EAGER moves the
  * load to context creation). Once loaded, the scratch stays resident on that device until the process
  * exits. Overlapping calls on one device race on the shared scratch: order them. particles_out must not

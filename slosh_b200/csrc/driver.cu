@@ -356,9 +356,7 @@ struct Ctx {
         sortb.vals[0] = dalloc<uint32_t>(cap, true);
         sortb.vals[1] = dalloc<uint32_t>(cap, true);
         sortb.perm = dalloc<uint32_t>(cap, true);
-        sortb.tile_hist_capacity = sort_tile_hist_size(cap);
-        sortb.tile_hist = dalloc<uint32_t>(sortb.tile_hist_capacity, true);
-        sortb.scan_tmp_capacity = sort_scan_tmp_size(cap, num_sort_keys);
+        sortb.scan_tmp_capacity = sort_scan_tmp_size(cap);
         sortb.scan_tmp = dalloc<uint32_t>(sortb.scan_tmp_capacity, true);
         if (p2g_gather_enabled()) {
             gather.rank = dalloc<uint32_t>(cap, true);

@@ -86,23 +86,20 @@ int launch_p2g_gather(const Dev& d, const Pass& p, const P2GGather& g, const slo
 struct SortBuffers {
     uint32_t* keys[2];
     uint32_t* vals[2];
-    uint32_t* tile_hist;     // 256 x num_tiles
     uint32_t* scan_tmp;      // block sums of the scans
-    uint32_t* counts;        // num_sort_keys
+    uint32_t* counts;        // num_sort_keys, or null
     uint32_t* offsets;       // num_sort_keys
     uint32_t* perm;          // capacity
     uint32_t* particle_count;
-    size_t tile_hist_capacity;
     size_t scan_tmp_capacity;
 };
 int3 sort_brick_dim(int3 grid);
 int launch_sort(const Dev& d, const SortBuffers& b, const slosh_particle_t* in, slosh_particle_t* out, uint32_t n,
                 uint32_t num_sort_keys, int3 sort_dim, cudaStream_t s);
-size_t sort_tile_hist_size(uint32_t capacity);
 // Exclusive prefix sum of n u32 (in place allowed); tmp holds exclusive_scan_tmp_size(n) words.
 int launch_exclusive_scan(const uint32_t* in, uint32_t* out, uint32_t n, uint32_t* tmp, cudaStream_t s);
 size_t exclusive_scan_tmp_size(uint32_t n);
-size_t sort_scan_tmp_size(uint32_t capacity, uint32_t num_sort_keys);
+size_t sort_scan_tmp_size(uint32_t capacity);
 
 // ---- MGPCG (SloshPressureMG.usf) ----
 struct MGLevel {

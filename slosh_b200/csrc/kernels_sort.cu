@@ -6,13 +6,20 @@
 // The reference ranks particles inside a key with an atomic counter, so its permutation depends on
 // thread timing. This sort is stable: it orders by key and, inside a key, by source slot -- the order
 // the reference produces when its atomics resolve in ascending thread order. It is an LSD radix sort of
-// (key, slot) pairs with 8-bit digits; each pass is reduce-then-scan:
-//   upsweep   per 4096-item tile, a shared-memory histogram of the digit (tile_hist[digit][tile]);
-//   scan      exclusive scan of tile_hist in digit-major order = each tile's first output position;
+// (key, slot) pairs whose digits split the key's bits evenly into the fewest passes of at most 10 bits (two
+// for 2^18 keys); each pass is reduce-then-scan:
+//   upsweep   per 4096-item tile, a shared-memory histogram of the digit (the first pass's by k_keys);
+//   scan      each tile's first output position of each digit: up to SORT_SMALL_TILES tiles every scatter CTA
+//             adds the whole histogram up for itself, beyond that an exclusive scan in digit-major order;
 //   scatter   each warp ranks its 512 contiguous items in order (warp match + per-warp counters), the
 //             per-warp counters are prefixed across warps, and items go to tile base + rank.
-// No step waits on another CTA. Per-key counts come from warp-aggregated atomics (integer, exact),
-// and their exclusive scan gives the key offsets and the live count.
+// One tile (n <= 4096) is sorted by one CTA in shared memory. The key offsets (and counts) are lower bounds in the
+// sorted keys, found beside the gather of the records. No step waits on another CTA.
+// A small sort is bound by its launches and their dependent loads: 3,001 records took 10 launches and 47 us with the
+// three-kernel scans and 8-bit digits, 200,003 records 15 launches and 83 us; now 2 launches and 12 us, 5 and 39 us.
+// 20.6 M records (2^18 keys): 1.22 ms with 3 passes of 8 bits and atomic counts, 0.80 ms with two of 10 and 9 bits.
+#include <algorithm>
+
 #include "kernels.h"
 
 namespace slosh {
@@ -42,56 +49,65 @@ __device__ __forceinline__ uint32_t tile_item(uint32_t tile, int r) {
     return tile * uint32_t(SORT_TILE) + uint32_t(warp * WARP_ITEMS + r * 32 + lane);
 }
 
-// Keys, per-key counts and the digit-0 tile histogram.
+constexpr int SORT_MAX_BITS = 10;                     // bits of a digit: 8 warps' counters of 1024 digits in 16 KB
+constexpr uint32_t SORT_SMALL_TILES = 64;             // tiles whose histograms every scatter CTA adds up itself
+
+// A tile's histogram of one digit: tile-major rows for few tiles (read whole by every scatter CTA), else digit-major
+// (scanned).
+__device__ __forceinline__ void store_hist(const uint32_t* hist, uint32_t* tile_hist, uint32_t num_tiles, uint32_t bins, bool small) {
+    for (uint32_t d = threadIdx.x; d < bins; d += SORT_THREADS)
+        tile_hist[small ? blockIdx.x * bins + d : d * num_tiles + blockIdx.x] = hist[d];
+}
+// Keys and the first digit's tile histogram.
 __global__ void __launch_bounds__(SORT_THREADS) k_keys(Dev d, const slosh_particle_t* __restrict__ particles, uint32_t n,
-                                                       uint32_t* __restrict__ keys, uint32_t* __restrict__ counts,
-                                                       uint32_t* __restrict__ tile_hist, uint32_t num_tiles, int3 sdim,
-                                                       uint32_t num_keys) {
-    __shared__ uint32_t hist[256];
-    hist[threadIdx.x] = 0u;
+                                                       uint32_t* __restrict__ keys, uint32_t* __restrict__ tile_hist,
+                                                       uint32_t num_tiles, uint32_t bins, bool small, int3 sdim, uint32_t num_keys) {
+    pdl_entry();
+    __shared__ uint32_t hist[1 << SORT_MAX_BITS];
+    for (uint32_t t = threadIdx.x; t < bins; t += SORT_THREADS) hist[t] = 0u;
     __syncthreads();
     const uint32_t tile = blockIdx.x;
-    const int lane = threadIdx.x & 31;
-#pragma unroll 4
+#pragma unroll 8
     for (int r = 0; r < SORT_ROUNDS; ++r) {
         const uint32_t i = tile_item(tile, r);
-        const bool valid = i < n;
-        uint32_t key = 0xFFFFFFFFu;
-        if (valid) {
-            key = sort_key_of(d, __ldg(reinterpret_cast<const float4*>(particles + i)), sdim, num_keys);
+        if (i < n) {
+            const uint32_t key = sort_key_of(d, __ldg(reinterpret_cast<const float4*>(particles + i)), sdim, num_keys);
             keys[i] = key;
-            atomicAdd(hist + (key & 0xFFu), 1u);
+            atomicAdd(hist + (key & (bins - 1u)), 1u);
         }
-        const uint32_t peers = __match_any_sync(0xFFFFFFFFu, key);
-        if (valid && lane == __ffs(peers) - 1) atomicAdd(counts + key, uint32_t(__popc(peers)));
     }
     __syncthreads();
-    tile_hist[threadIdx.x * num_tiles + tile] = hist[threadIdx.x];
+    store_hist(hist, tile_hist, num_tiles, bins, small);
 }
 
-__global__ void __launch_bounds__(SORT_THREADS) k_upsweep(const uint32_t* __restrict__ keys, uint32_t n, uint32_t* __restrict__ tile_hist,
-                                                          uint32_t num_tiles, uint32_t shift) {
-    __shared__ uint32_t hist[256];
-    hist[threadIdx.x] = 0u;
+__global__ void __launch_bounds__(SORT_THREADS) k_upsweep(const uint32_t* keys, uint32_t n, uint32_t* __restrict__ tile_hist,
+                                                          uint32_t num_tiles, uint32_t bins, bool small, uint32_t shift) {
+    pdl_entry();
+    __shared__ uint32_t hist[1 << SORT_MAX_BITS];
+    for (uint32_t t = threadIdx.x; t < bins; t += SORT_THREADS) hist[t] = 0u;
     __syncthreads();
     const uint32_t tile = blockIdx.x;
-#pragma unroll 4
+#pragma unroll 8
     for (int r = 0; r < SORT_ROUNDS; ++r) {
         const uint32_t i = tile_item(tile, r);
-        if (i < n) atomicAdd(hist + ((__ldg(keys + i) >> shift) & 0xFFu), 1u);
+        if (i < n) atomicAdd(hist + ((keys[i] >> shift) & (bins - 1u)), 1u);
     }
     __syncthreads();
-    tile_hist[threadIdx.x * num_tiles + tile] = hist[threadIdx.x];
+    store_hist(hist, tile_hist, num_tiles, bins, small);
 }
 
-// Stable scatter of one digit. vals_in == nullptr means the identity (source slot = item index);
-// keys_out == nullptr skips writing keys (last pass).
-__global__ void __launch_bounds__(SORT_THREADS) k_scatter(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
-                                                          uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, uint32_t n,
-                                                          const uint32_t* __restrict__ tile_scan, uint32_t num_tiles, uint32_t shift) {
-    __shared__ uint32_t whist[SORT_WARPS][256];
-    for (int t = threadIdx.x; t < SORT_WARPS * 256; t += SORT_THREADS) (&whist[0][0])[t] = 0u;
-    __syncthreads();
+__device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* s_warp, uint32_t* total);
+
+// Stable scatter of one digit. vals_in == nullptr means the identity (source slot = item index). tile_hist holds the
+// tiles' histograms (small) or their scan.
+__global__ void __launch_bounds__(SORT_THREADS) k_scatter(const uint32_t* keys_in, const uint32_t* vals_in, uint32_t* keys_out,
+                                                          uint32_t* vals_out, uint32_t n, const uint32_t* tile_hist, uint32_t num_tiles,
+                                                          uint32_t bins, bool small, uint32_t shift) {
+    pdl_entry();
+    __shared__ uint16_t whist[SORT_WARPS][1 << SORT_MAX_BITS];  // a warp's counts, then its first place in the tile
+    __shared__ uint32_t first[1 << SORT_MAX_BITS];              // the tile's first output position
+    __shared__ uint32_t total[1 << SORT_MAX_BITS];
+    __shared__ uint32_t s_warp[33];
     const uint32_t tile = blockIdx.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t lt_mask = (1u << lane) - 1u;
@@ -99,26 +115,59 @@ __global__ void __launch_bounds__(SORT_THREADS) k_scatter(const uint32_t* __rest
 #pragma unroll
     for (int r = 0; r < SORT_ROUNDS; ++r) {
         const uint32_t i = tile_item(tile, r);
-        const bool valid = i < n;
-        key[r] = valid ? __ldg(keys_in + i) : 0u;
-        val[r] = valid ? (vals_in ? __ldg(vals_in + i) : i) : 0u;
-        const uint32_t digit = valid ? ((key[r] >> shift) & 0xFFu) : 0xFFFFFFFFu;
+        key[r] = i < n ? keys_in[i] : 0u;
+        val[r] = i < n ? (vals_in ? vals_in[i] : i) : 0u;
+    }
+    for (uint32_t t = threadIdx.x; t < bins; t += SORT_THREADS) first[t] = total[t] = 0u;
+#pragma unroll
+    for (int w = 0; w < SORT_WARPS; ++w)
+        for (uint32_t t = threadIdx.x; t < bins; t += SORT_THREADS) whist[w][t] = 0u;
+    __syncthreads();
+    if (small) {
+        const uint32_t words = num_tiles * bins;
+#pragma unroll 8
+        for (uint32_t t = threadIdx.x; t < words; t += SORT_THREADS) {
+            const uint32_t v = tile_hist[t], dgt = t & (bins - 1u);
+            if (v != 0u) {
+                atomicAdd(total + dgt, v);
+                if (t < tile * bins) atomicAdd(first + dgt, v);
+            }
+        }
+    } else {
+        for (uint32_t t = threadIdx.x; t < bins; t += SORT_THREADS) first[t] = tile_hist[t * num_tiles + tile];
+    }
+#pragma unroll
+    for (int r = 0; r < SORT_ROUNDS; ++r) {
+        const bool valid = tile_item(tile, r) < n;
+        const uint32_t digit = valid ? ((key[r] >> shift) & (bins - 1u)) : 0xFFFFFFFFu;
         const uint32_t peers = __match_any_sync(0xFFFFFFFFu, digit);
         uint32_t before = 0u;
         if (valid) before = whist[warp][digit];
         __syncwarp();
-        if (valid && lane == __ffs(peers) - 1) whist[warp][digit] = before + uint32_t(__popc(peers));
+        if (valid && lane == __ffs(int(peers)) - 1) whist[warp][digit] = uint16_t(before + uint32_t(__popc(peers)));
         __syncwarp();
         rank[r] = valid ? before + uint32_t(__popc(peers & lt_mask)) : 0xFFFFFFFFu;
     }
     __syncthreads();
-    {
-        const uint32_t dgt = threadIdx.x;
-        uint32_t run = tile_scan[dgt * num_tiles + tile];
+    if (small) {  // the digits' exclusive scan: thread t takes the digits from t * per
+        const uint32_t per = (bins + SORT_THREADS - 1u) / SORT_THREADS, d0 = threadIdx.x * per;
+        uint32_t v = 0u;
+        for (uint32_t j = 0; j < per; ++j)
+            if (d0 + j < bins) v += total[d0 + j];
+        uint32_t all;
+        uint32_t run = block_excl_scan(v, s_warp, &all);
+        for (uint32_t j = 0; j < per; ++j)
+            if (d0 + j < bins) {
+                first[d0 + j] += run;
+                run += total[d0 + j];
+            }
+    }
+    for (uint32_t dgt = threadIdx.x; dgt < bins; dgt += SORT_THREADS) {
+        uint32_t run = 0u;
 #pragma unroll
         for (int w = 0; w < SORT_WARPS; ++w) {
             const uint32_t t = whist[w][dgt];
-            whist[w][dgt] = run;
+            whist[w][dgt] = uint16_t(run);
             run += t;
         }
     }
@@ -126,25 +175,129 @@ __global__ void __launch_bounds__(SORT_THREADS) k_scatter(const uint32_t* __rest
 #pragma unroll
     for (int r = 0; r < SORT_ROUNDS; ++r) {
         if (rank[r] == 0xFFFFFFFFu) continue;
-        const uint32_t dst = whist[warp][(key[r] >> shift) & 0xFFu] + rank[r];
-        if (keys_out) keys_out[dst] = key[r];
+        const uint32_t dgt = (key[r] >> shift) & (bins - 1u);
+        const uint32_t dst = first[dgt] + whist[warp][dgt] + rank[r];
+        keys_out[dst] = key[r];
         vals_out[dst] = val[r];
     }
 }
 
-// Gather of the 48-byte records in sorted order; perm keeps the source slot of every output.
-__global__ void k_gather(const slosh_particle_t* __restrict__ in, slosh_particle_t* __restrict__ out, const uint32_t* __restrict__ vals,
-                         uint32_t* __restrict__ perm, uint32_t n) {
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    const uint32_t src = __ldg(vals + j);
-    const float4* s = reinterpret_cast<const float4*>(in + src);
-    float4* o = reinterpret_cast<float4*>(out + j);
-    const float4 a = __ldg(s), b = __ldg(s + 1), c = __ldg(s + 2);
-    o[0] = a;
-    o[1] = b;
-    o[2] = c;
-    perm[j] = src;
+// The whole radix sort of one tile by one CTA of 1024 threads, 4 items each, in shared memory; 8-bit digits.
+constexpr int TILE_THREADS = 1024, TILE_WARPS = TILE_THREADS / 32, TILE_ROUNDS = SORT_TILE / TILE_THREADS;
+__global__ void __launch_bounds__(TILE_THREADS) k_sort_tile(Dev d, const slosh_particle_t* __restrict__ particles, uint32_t n,
+                                                            uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, int bits,
+                                                            int3 sdim, uint32_t num_keys) {
+    pdl_entry();
+    __shared__ uint16_t whist[TILE_WARPS][256];
+    __shared__ uint32_t s_keys[SORT_TILE];
+    __shared__ uint16_t s_vals[SORT_TILE];
+    __shared__ uint32_t s_warp[33];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t lt_mask = (1u << lane) - 1u;
+    uint32_t key[TILE_ROUNDS], val[TILE_ROUNDS], rank[TILE_ROUNDS];
+    auto item = [&](int r) { return uint32_t(warp * 32 * TILE_ROUNDS + r * 32 + lane); };
+#pragma unroll
+    for (int r = 0; r < TILE_ROUNDS; ++r) {
+        const uint32_t i = item(r);
+        key[r] = i < n ? sort_key_of(d, __ldg(reinterpret_cast<const float4*>(particles + i)), sdim, num_keys) : 0u;
+        val[r] = i;
+    }
+    for (int shift = 0; shift < bits || shift == 0; shift += 8) {
+        for (uint32_t t = threadIdx.x; t < uint32_t(TILE_WARPS) * 128u; t += TILE_THREADS) reinterpret_cast<uint32_t*>(&whist[0][0])[t] = 0u;
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < TILE_ROUNDS; ++r) {
+            const bool valid = item(r) < n;
+            const uint32_t digit = valid ? ((key[r] >> shift) & 0xFFu) : 0xFFFFFFFFu;
+            const uint32_t peers = __match_any_sync(0xFFFFFFFFu, digit);
+            uint32_t before = 0u;
+            if (valid) before = whist[warp][digit];
+            __syncwarp();
+            if (valid && lane == __ffs(int(peers)) - 1) whist[warp][digit] = uint16_t(before + uint32_t(__popc(peers)));
+            __syncwarp();
+            rank[r] = before + uint32_t(__popc(peers & lt_mask));
+        }
+        __syncthreads();
+        uint32_t sum = 0u;
+        if (threadIdx.x < 256u) {
+#pragma unroll 8
+            for (int w = 0; w < TILE_WARPS; ++w) sum += whist[w][threadIdx.x];
+        }
+        uint32_t all;
+        uint32_t run = block_excl_scan(sum, s_warp, &all);
+        if (threadIdx.x < 256u) {
+#pragma unroll 8
+            for (int w = 0; w < TILE_WARPS; ++w) {
+                const uint32_t t = whist[w][threadIdx.x];
+                whist[w][threadIdx.x] = uint16_t(run);
+                run += t;
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < TILE_ROUNDS; ++r) {
+            if (item(r) >= n) continue;
+            const uint32_t dst = whist[warp][(key[r] >> shift) & 0xFFu] + rank[r];
+            s_keys[dst] = key[r];
+            s_vals[dst] = uint16_t(val[r]);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < TILE_ROUNDS; ++r) {
+            const uint32_t i = item(r);
+            if (i >= n) continue;
+            key[r] = s_keys[i];
+            val[r] = s_vals[i];
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < TILE_ROUNDS; ++r) {
+        const uint32_t i = item(r);
+        if (i >= n) continue;
+        keys_out[i] = key[r];
+        vals_out[i] = val[r];
+    }
+}
+
+// Gather of the 48-byte records in sorted order (perm keeps the source slot of every output), and for thread k < num_keys
+// the key's offset: the number of sorted keys below k. The last key is the dead records', so its offset is the live count.
+// counts may be null.
+__device__ __forceinline__ uint32_t lower_bound_key(const uint32_t* keys, uint32_t n, uint32_t k) {
+    uint32_t lo = 0u, hi = n;
+    while (lo < hi) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (keys[mid] < k) lo = mid + 1u;
+        else hi = mid;
+    }
+    return lo;
+}
+__global__ void __launch_bounds__(256) k_gather(const slosh_particle_t* __restrict__ in, slosh_particle_t* __restrict__ out, const uint32_t* keys,
+                                                const uint32_t* vals, uint32_t* __restrict__ perm, uint32_t n,
+                                                uint32_t* __restrict__ offsets, uint32_t* __restrict__ counts, uint32_t num_keys,
+                                                uint32_t* __restrict__ pc) {
+    pdl_entry();
+    const uint32_t j = blockIdx.x * 256u + threadIdx.x;
+    if (j < n) {
+        const uint32_t src = vals[j];
+        const float4* s = reinterpret_cast<const float4*>(in + src);
+        float4* o = reinterpret_cast<float4*>(out + j);
+        const float4 a = __ldg(s), b = __ldg(s + 1), c = __ldg(s + 2);
+        o[0] = a;
+        o[1] = b;
+        o[2] = c;
+        perm[j] = src;
+    }
+    if ((j & ~31u) >= num_keys) return;
+    const uint32_t at = lower_bound_key(keys, n, min(j, num_keys));
+    if (j < num_keys) {
+        offsets[j] = at;
+        if (j == num_keys - 1u) pc[0] = at;
+    }
+    if (counts) {  // warp-uniform; the next lane's offset, the last lane's by another search
+        uint32_t next = __shfl_down_sync(0xFFFFFFFFu, at, 1);
+        if ((j & 31u) == 31u || j + 1u >= num_keys) next = j + 1u < num_keys ? lower_bound_key(keys, n, j + 1u) : n;
+        if (j < num_keys) counts[j] = next - at;
+    }
 }
 
 // ---- exclusive scan of u32 (three kernels, in place allowed) ----------------------------------------
@@ -259,10 +412,6 @@ int exclusive_scan(const uint32_t* in, uint32_t* out, uint32_t n, uint32_t* tmp,
     return 3;
 }
 
-__global__ void k_live_count(const uint32_t* offsets, uint32_t num_keys, uint32_t* pc) {
-    pc[0] = offsets[num_keys - 1u];
-}
-
 }  // namespace
 
 int launch_exclusive_scan(const uint32_t* in, uint32_t* out, uint32_t n, uint32_t* tmp, cudaStream_t s) {
@@ -272,50 +421,42 @@ size_t exclusive_scan_tmp_size(uint32_t n) { return (size_t(n) + SCAN_TILE - 1) 
 
 int3 sort_brick_dim(int3 g) { return make_int3((g.x + 3) / 4, (g.y + 3) / 4, (g.z + 3) / 4); }
 
-size_t sort_tile_hist_size(uint32_t capacity) {
-    const size_t tiles = (size_t(capacity) + SORT_TILE - 1) / SORT_TILE;
-    return 256 * (tiles > 0 ? tiles : 1);
-}
-size_t sort_scan_tmp_size(uint32_t capacity, uint32_t num_sort_keys) {
-    const size_t a = (sort_tile_hist_size(capacity) + SCAN_TILE - 1) / SCAN_TILE;
-    const size_t b = (size_t(num_sort_keys) + SCAN_TILE - 1) / SCAN_TILE;
-    return (a > b ? a : b) + 1;
+// Block sums of the largest scan: the tiles' histograms, at most a quarter word per particle and a row.
+size_t sort_scan_tmp_size(uint32_t capacity) {
+    return (size_t(capacity) / 4 + (size_t(1) << SORT_MAX_BITS) + SCAN_TILE - 1) / SCAN_TILE + 1;
 }
 
 int launch_sort(const Dev& d, const SortBuffers& b, const slosh_particle_t* in, slosh_particle_t* out, uint32_t n,
                 uint32_t num_keys, int3 sdim, cudaStream_t s) {
     int launches = 0;
-    cudaMemsetAsync(b.counts, 0, sizeof(uint32_t) * num_keys, s);
-    if (n == 0) {
-        launches += exclusive_scan(b.counts, b.offsets, num_keys, b.scan_tmp, s);
-        k_live_count<<<1, 1, 0, s>>>(b.offsets, num_keys, b.particle_count);
-        return launches + 1;
-    }
-    const uint32_t num_tiles = (n + uint32_t(SORT_TILE) - 1u) / uint32_t(SORT_TILE);
-    const uint32_t hist_n = 256u * num_tiles;
     uint32_t bits = 0;
     while ((1u << bits) < num_keys && bits < 32) ++bits;  // keys are < num_keys
-    const int passes = bits <= 8 ? 1 : int((bits + 7) / 8);
-    k_keys<<<num_tiles, SORT_THREADS, 0, s>>>(d, in, n, b.keys[0], b.counts, b.tile_hist, num_tiles, sdim, num_keys);
-    ++launches;
+    const uint32_t num_tiles = (n + uint32_t(SORT_TILE) - 1u) / uint32_t(SORT_TILE);
     int cur = 0;
-    for (int pass = 0; pass < passes; ++pass) {
-        const uint32_t shift = uint32_t(pass) * 8u;
-        if (pass > 0) {
-            k_upsweep<<<num_tiles, SORT_THREADS, 0, s>>>(b.keys[cur], n, b.tile_hist, num_tiles, shift);
-            ++launches;
-        }
-        launches += exclusive_scan(b.tile_hist, b.tile_hist, hist_n, b.scan_tmp, s);
-        const bool last = pass == passes - 1;
-        k_scatter<<<num_tiles, SORT_THREADS, 0, s>>>(b.keys[cur], pass == 0 ? nullptr : b.vals[cur], last ? nullptr : b.keys[cur ^ 1],
-                                                     b.vals[cur ^ 1], n, b.tile_hist, num_tiles, shift);
+    if (num_tiles == 1u) {
+        launch_k(k_sort_tile, 1, TILE_THREADS, 0, s, d, in, n, b.keys[0], b.vals[0], int(bits), sdim, num_keys);
         ++launches;
-        cur ^= 1;
+    } else if (num_tiles > 1u) {
+        const int passes = std::max(1, int((bits + SORT_MAX_BITS - 1) / SORT_MAX_BITS));
+        const bool small = num_tiles <= SORT_SMALL_TILES;
+        uint32_t* hist = b.perm;  // 2^10 words a tile of 4096 fit the permutation, which only the gather writes
+        uint32_t shift = 0;
+        for (int pass = 0; pass < passes; ++pass) {
+            const uint32_t width = (bits - shift + uint32_t(passes - pass) - 1u) / uint32_t(passes - pass);
+            const uint32_t bins = 1u << std::max(width, 1u);
+            if (pass == 0) launch_k(k_keys, num_tiles, SORT_THREADS, 0, s, d, in, n, b.keys[0], hist, num_tiles, bins, small, sdim, num_keys);
+            else launch_k(k_upsweep, num_tiles, SORT_THREADS, 0, s, b.keys[cur], n, hist, num_tiles, bins, small, shift);
+            ++launches;
+            if (!small) launches += exclusive_scan(hist, hist, bins * num_tiles, b.scan_tmp, s);
+            launch_k(k_scatter, num_tiles, SORT_THREADS, 0, s, b.keys[cur], pass == 0 ? nullptr : b.vals[cur], b.keys[cur ^ 1], b.vals[cur ^ 1],
+                     n, hist, num_tiles, bins, small, shift);
+            ++launches;
+            cur ^= 1;
+            shift += width;
+        }
     }
-    k_gather<<<(n + 255u) / 256u, 256, 0, s>>>(in, out, b.vals[cur], b.perm, n);
-    ++launches;
-    launches += exclusive_scan(b.counts, b.offsets, num_keys, b.scan_tmp, s);
-    k_live_count<<<1, 1, 0, s>>>(b.offsets, num_keys, b.particle_count);
+    launch_k(k_gather, (std::max(n, num_keys) + 255u) / 256u, 256, 0, s, in, out, b.keys[cur], b.vals[cur], b.perm, n, b.offsets, b.counts,
+             num_keys, b.particle_count);
     return launches + 1;
 }
 

@@ -4,7 +4,7 @@
 // allocates. This entry point runs the same kernels (launch_sort: keys, digit histograms, scans, stable
 // scatter, gather) on particle arrays that the caller owns, without a context and without allocating
 // anything: its scratch is the one static device array below, sized for at most
-// SLOSH_STATIC_SORT_MAX_PARTICLES particles and SLOSH_STATIC_SORT_MAX_KEYS sort keys (7.4 MB per device).
+// SLOSH_STATIC_SORT_MAX_PARTICLES particles and SLOSH_STATIC_SORT_MAX_KEYS sort keys (6.3 MB per device).
 //
 // Who cannot allocate here, and why:
 //   * an engine that reserves its device memory once at start-up and afterwards hands the simulation
@@ -30,8 +30,7 @@
 // threads, with nothing ordering them -- race on it and corrupt each other's results. Issue them on one
 // stream, or order them with events or a lock.
 //
-// What must start at zero: only the per-key counts, which launch_sort clears on the stream at the start of
-// every call; every other scratch word is written before it is read within the call.
+// Nothing must start at zero: every scratch word is written before it is read within the call.
 #include <cuda.h>  // CUcontext and CUresult only: the driver calls are fetched at run time
 
 #include <cmath>
@@ -51,13 +50,12 @@ constexpr uint32_t kMaxParticles = SLOSH_STATIC_SORT_MAX_PARTICLES;
 constexpr uint32_t kMaxKeys = SLOSH_STATIC_SORT_MAX_KEYS;
 constexpr size_t kAlignWords = 64;  // 256-byte sub-buffers
 constexpr size_t round_up(size_t w) { return (w + kAlignWords - 1) / kAlignWords * kAlignWords; }
-// Tile histogram: 256 digits x one 4096-particle tile; scan block sums: one per 4096 scanned words.
-constexpr size_t kTileHistWords = round_up(256 * ((size_t(kMaxParticles) + 4095) / 4096));
-constexpr size_t kScanTmpWords = round_up(((kTileHistWords > kMaxKeys ? kTileHistWords : kMaxKeys) + 4095) / 4096 + 1);
+// Scan block sums: one per 4096 words of the tiles' histograms (launch_sort keeps those in the permutation).
+constexpr size_t kScanTmpWords = round_up((size_t(kMaxParticles) / 4 + 1024 + 4095) / 4096 + 1);
 constexpr size_t kParticleWords = round_up(kMaxParticles);
 constexpr size_t kKeyWords = round_up(kMaxKeys);
-// keys[2], vals[2], perm | counts, offsets | tile histogram | scan sums | live count
-constexpr size_t kScratchWords = 5 * kParticleWords + 2 * kKeyWords + kTileHistWords + kScanTmpWords + kAlignWords;
+// keys[2], vals[2], perm | offsets | scan sums | live count
+constexpr size_t kScratchWords = 5 * kParticleWords + kKeyWords + kScanTmpWords + kAlignWords;
 
 static __device__ __align__(256) uint32_t g_sort_scratch[kScratchWords];
 
@@ -195,14 +193,12 @@ SLOSH_API slosh_status slosh_sort_particles_static(const slosh_particle_t* parti
     b.vals[0] = w; w += kParticleWords;
     b.vals[1] = w; w += kParticleWords;
     b.perm = perm_out ? perm_out : w; w += kParticleWords;
-    b.counts = w; w += kKeyWords;
+    b.counts = nullptr;  // not an output of this entry point
     b.offsets = key_offsets_out ? key_offsets_out : w; w += kKeyWords;
-    b.tile_hist = w; w += kTileHistWords;
     b.scan_tmp = w; w += kScanTmpWords;
     b.particle_count = live_count_out ? live_count_out : w;
-    b.tile_hist_capacity = kTileHistWords;
     b.scan_tmp_capacity = kScanTmpWords;
-    if (sort_tile_hist_size(count) > kTileHistWords || sort_scan_tmp_size(count, num_keys) > kScanTmpWords)
+    if (sort_scan_tmp_size(count) > kScanTmpWords)
         return fail(SLOSH_ERR_CAPACITY, std::string(fn) + "internal scratch layout too small");
 
     // The sort kernels read only the grid extents and the inverse cell size of the device view.
