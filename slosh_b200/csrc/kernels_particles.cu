@@ -660,6 +660,12 @@ __device__ __forceinline__ float sample_component(const Dev& d, int axis, float3
     }
     return lerp3(u, s.fx, s.fy, s.fz, d.inv_h, false, nullptr);
 }
+// The displacement of at most half a cell, in metres (Slosh.usf:848-853).
+__device__ __forceinline__ float3 displacement_step(const Dev& d, float3 v) {
+    const float len = len3(v);
+    const float3 dd = len > 0.5f ? mul3s(v, 0.5f / len) : v;
+    return mul3s(dd, d.h);
+}
 // SampleDensityDisplacement (Slosh.usf:830-854).
 __device__ __forceinline__ float3 sample_displacement(const Dev& d, float3 xp, const float* __restrict__ disp) {
     float out[3];
@@ -673,11 +679,96 @@ __device__ __forceinline__ float3 sample_displacement(const Dev& d, float3 xp, c
         for (int o = 0; o < 8; ++o) u[o] = disp[idx[o]];
         out[axis] = lerp3(u, s.fx, s.fy, s.fz, d.inv_h, false, nullptr);
     }
-    const float3 v = make_float3(out[0], out[1], out[2]);
-    const float len = len3(v);
-    const float3 dd = len > 0.5f ? mul3s(v, 0.5f / len) : v;
-    return mul3s(dd, d.h);
+    return displacement_step(d, make_float3(out[0], out[1], out[2]));
 }
+
+// Where G2P reads the velocity (and displacement) field: in global memory through the brick table.
+struct GlobalField {
+    const float* __restrict__ vel;
+    const float* __restrict__ disp;
+    __device__ __forceinline__ void gather(const Dev& d, const Pass& p, float3 x, float3& u, float3& dsum, float3& dw, float3 (&g)[3]) const {
+        gather_component(d, p, 0, x, vel, u.x, dsum.x, dw.x, g[0]);
+        gather_component(d, p, 1, x, vel, u.y, dsum.y, dw.y, g[1]);
+        gather_component(d, p, 2, x, vel, u.z, dsum.z, dw.z, g[2]);
+    }
+    __device__ __forceinline__ float3 sample(const Dev& d, float3 x, float3 fallback, bool check) const {
+        return make_float3(sample_component(d, 0, x, fallback.x, check, vel), sample_component(d, 1, x, fallback.y, check, vel),
+                           sample_component(d, 2, x, fallback.z, check, vel));
+    }
+    __device__ __forceinline__ float3 displacement(const Dev& d, float3 x) const { return sample_displacement(d, x, disp); }
+};
+
+// The same from a shared-memory tile: the three components (and the displacement's) at the nodes of a box of cells.
+// Tile index of node n: (n.x - origin.x) + sy (n.y - origin.y) + sz (n.z - origin.z). A position whose stencils leave
+// the tile or the grid (where the global form clamps its nodes), or that needs the face flags, is read from global memory.
+constexpr int G2P_TILE_NODES = 2040;  // six planes stay below the 48 KB that need no attribute
+struct TileField {
+    GlobalField global;
+    const float* tile;  // [3 or 6][G2P_TILE_NODES]; null: the box did not fit
+    int3 origin, dim;
+    int sy, sz;
+    // Of a position: per axis the stencil's first node for a face on the axis (0) and beside it (1) and the fractions; the
+    // bits of the global form's stencil_of. False when a node lies outside the tile (whose nodes are inside the grid).
+    struct At {
+        int b[3][2];
+        float f[3][2];
+    };
+    __device__ __forceinline__ bool at(const Dev& d, float3 x, At& q) const {
+        if (!tile) return false;
+        const float g[3] = {x.x * d.inv_h, x.y * d.inv_h, x.z * d.inv_h};
+        const int o[3] = {origin.x, origin.y, origin.z}, n[3] = {dim.x, dim.y, dim.z};
+        bool in = true;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+#pragma unroll
+            for (int v = 0; v < 2; ++v) {
+                const float gv = g[a] - (v ? 0.5f : 0.0f), fl = floorf(gv);
+                q.b[a][v] = int(fl) - o[a];
+                q.f[a][v] = gv - fl;
+            }
+            in = in && q.b[a][1] >= 0 && q.b[a][0] < n[a] - 1;  // the stencil beside starts no later and ends no later
+        }
+        return in;
+    }
+    __device__ __forceinline__ void values(const At& q, int axis, const float* plane, float (&u)[8], float& fx, float& fy, float& fz) const {
+        const int vx = axis == 0 ? 0 : 1, vy = axis == 1 ? 0 : 1, vz = axis == 2 ? 0 : 1;
+        const float* t = plane + q.b[0][vx] + sy * q.b[1][vy] + sz * q.b[2][vz];
+        u[0] = t[0]; u[1] = t[1];
+        u[2] = t[sy]; u[3] = t[sy + 1];
+        u[4] = t[sz]; u[5] = t[sz + 1];
+        u[6] = t[sz + sy]; u[7] = t[sz + sy + 1];
+        fx = q.f[0][vx]; fy = q.f[1][vy]; fz = q.f[2][vz];
+    }
+    __device__ __forceinline__ float value(const Dev& d, const At& q, int axis, const float* planes, bool grad, float3* g) const {
+        float u[8], fx, fy, fz;
+        values(q, axis, planes + axis * G2P_TILE_NODES, u, fx, fy, fz);
+        return lerp3(u, fx, fy, fz, d.inv_h, grad, g);
+    }
+    // APIC only: the FLIP sums need the flags and the old velocities
+    __device__ __forceinline__ void gather(const Dev& d, const Pass& p, float3 x, float3& u, float3& dsum, float3& dw, float3 (&g)[3]) const {
+        At q;
+        if (!at(d, x, q)) {
+            global.gather(d, p, x, u, dsum, dw, g);
+            return;
+        }
+        dsum = dw = make_float3(0.0f, 0.0f, 0.0f);
+        u.x = value(d, q, 0, tile, true, &g[0]);
+        u.y = value(d, q, 1, tile, true, &g[1]);
+        u.z = value(d, q, 2, tile, true, &g[2]);
+    }
+    __device__ __forceinline__ float3 sample(const Dev& d, float3 x, float3 fallback, bool check) const {
+        At q;
+        if (check || !at(d, x, q)) return global.sample(d, x, fallback, check);
+        return make_float3(value(d, q, 0, tile, false, nullptr), value(d, q, 1, tile, false, nullptr), value(d, q, 2, tile, false, nullptr));
+    }
+    __device__ __forceinline__ float3 displacement(const Dev& d, float3 x) const {
+        At q;
+        if (!at(d, x, q)) return global.displacement(d, x);
+        const float* planes = tile + 3 * G2P_TILE_NODES;
+        return displacement_step(d, make_float3(value(d, q, 0, planes, false, nullptr), value(d, q, 1, planes, false, nullptr),
+                                                value(d, q, 2, planes, false, nullptr)));
+    }
+};
 
 constexpr int G2P_THREADS = 256;
 // The new particle record is written once and read again only by the next substep's passes, after the grid
@@ -691,32 +782,33 @@ __device__ __forceinline__ void g2p_store(slosh_particle_t* out, uint32_t i, flo
     __stcs(reinterpret_cast<uint4*>(v + 2), make_uint4(c[1], c[2], c[3], c[4]));
 }
 
-// AdvectParticle + G2PAdvectCS (Slosh.usf:1452-1678). Each thread gathers its stencils straight from the brick
-// pool through the brick table; the particles are brick-sorted, so a warp's gathers hit the same few bricks in L1.
-// Staging each CTA's particle box of face velocities in shared memory first (24 KB tile, 3-cell margin) measured
-// slower (1.22 ms against 0.99 ms per 256^3 substep): the fill reads more nodes than the stencils touch.
-template <int MINB>
-__global__ void __launch_bounds__(G2P_THREADS, MINB) k_g2p(Dev d, Pass p, slosh_particle_t* __restrict__ particles, uint32_t n,
-                                                     const float* __restrict__ vel, const float* __restrict__ disp,
-                                                     uint32_t apply_density) {
-    const uint32_t i = blockIdx.x * G2P_THREADS + threadIdx.x;
-    uint32_t brick = NO_BRICK;
-    uint32_t speed_bits = 0u;
-    if (i < n) {
-        float4 ra, rb;
-        uint4 rc;
-        load_particle_raw(particles, i, ra, rb, rc);
-        ParticleF P = unpack_particle(ra, rb, rc);
-        if (!is_dead_age(P.age)) {
+// AdvectParticle + G2PAdvectCS (Slosh.usf:1452-1678) of live particle i at (pos, age). Returns its brick and speed.
+template <class Field>
+__device__ __forceinline__ void g2p_particle(const Dev& d, const Pass& p, slosh_particle_t* __restrict__ particles, uint32_t i, float4 ra,
+                                             const Field& field, bool apply_density, uint32_t& brick, uint32_t& speed_bits) {
+    struct {
+        float3 pos, vel;
+        float age;
+    } P;
+    P.pos = make_float3(ra.x, ra.y, ra.z);
+    P.age = ra.w;
+    // the old velocity: FLIP's, and the ballistic fallback's (loaded there by the few particles in it)
+    auto old_vel = [&]() {
+        const float4 rb = __ldg(reinterpret_cast<const float4*>(particles + i) + 1);
+        return make_float3(rb.x, rb.y, rb.z);
+    };
+    if (p.use_apic == 0u) P.vel = old_vel();
+    {
+        {
             const float h = d.h, inv_h = d.inv_h, dt = p.dt;
             const float lo = h * 1.01f;
             const float3 hi = make_float3((float(d.grid.x) - 1.01f) * h, (float(d.grid.y) - 1.01f) * h, (float(d.grid.z) - 1.01f) * h);
             float3 pic, delta, dw, gx, gy, gz;
             const uint32_t zero_c = pack_half2(0.0f, 0.0f);
             uint32_t cw[5] = {zero_c, zero_c, zero_c, zero_c, zero_c};  // the packed APIC rows (zero for PIC/FLIP)
-            gather_component(d, p, 0, P.pos, vel, pic.x, delta.x, dw.x, gx);
-            gather_component(d, p, 1, P.pos, vel, pic.y, delta.y, dw.y, gy);
-            gather_component(d, p, 2, P.pos, vel, pic.z, delta.z, dw.z, gz);
+            float3 grad[3];
+            field.gather(d, p, P.pos, pic, delta, dw, grad);
+            gx = grad[0]; gy = grad[1]; gz = grad[2];
             float3 nv;
             if (p.use_apic) {
                 nv = pic;
@@ -743,15 +835,14 @@ __global__ void __launch_bounds__(G2P_THREADS, MINB) k_g2p(Dev d, Pass p, slosh_
             float3 v2 = v1;
             if (mid_cells < 2.0f) {
                 const bool check = mid_cells > 1.0f;
-                const float3 sv = make_float3(sample_component(d, 0, mid, v1.x, check, vel), sample_component(d, 1, mid, v1.y, check, vel),
-                                              sample_component(d, 2, mid, v1.z, check, vel));
+                const float3 sv = field.sample(d, mid, v1, check);
                 const float t = saturatef(mid_cells - 1.0f);
                 v2 = make_float3(sv.x + t * (v1.x - sv.x), sv.y + t * (v1.y - sv.y), sv.z + t * (v1.z - sv.z));
             }
             float3 x = addf3(P.pos, scale3(dt, v2));
             if (apply_density) {
                 const float3 cpos = make_float3(clampf(P.pos.x, lo, hi.x), clampf(P.pos.y, lo, hi.y), clampf(P.pos.z, lo, hi.z));
-                x = addf3(x, sample_displacement(d, cpos, disp));
+                x = addf3(x, field.displacement(d, cpos));
             }
             // Pool exhausted: ballistic.
             const int3 pcell = make_int3(clampi(int(floorf(P.pos.x * inv_h)), 0, d.grid.x - 1),
@@ -759,7 +850,7 @@ __global__ void __launch_bounds__(G2P_THREADS, MINB) k_g2p(Dev d, Pass p, slosh_
                                          clampi(int(floorf(P.pos.z * inv_h)), 0, d.grid.z - 1));
             if (is_null_cell(cell_index(d, pcell))) {
                 const float3 g = make_float3(p.gravity[0], p.gravity[1], p.gravity[2]);
-                nv = addf3(P.vel, mul3s(g, dt));
+                nv = addf3(old_vel(), mul3s(g, dt));
                 x = addf3(P.pos, scale3(dt, nv));
 #pragma unroll
                 for (int k = 0; k < 5; ++k) cw[k] = zero_c;
@@ -860,11 +951,92 @@ __global__ void __launch_bounds__(G2P_THREADS, MINB) k_g2p(Dev d, Pass p, slosh_
             }
         }
     }
-    // Touch flags: sorted particles mostly share bricks, so only the first lane of each run writes.
+}
+// Ends a G2P CTA: touch flags and the fastest particle. Sorted particles mostly share bricks, so only the first lane of
+// each run writes.
+__device__ __forceinline__ void g2p_finish(const Dev& d, uint32_t brick, uint32_t speed_bits) {
     const uint32_t prev = __shfl_up_sync(0xFFFFFFFFu, brick, 1);
     if (brick != NO_BRICK && ((threadIdx.x & 31) == 0 || prev != brick)) d.brick_touch[brick] = 1u;
     speed_bits = __reduce_max_sync(0xFFFFFFFFu, speed_bits);
     if ((threadIdx.x & 31) == 0 && speed_bits) atomicMax(d.stats + 0, speed_bits);
+}
+
+// Stencils straight from the brick pool through the brick table (PIC/FLIP, whose sums also need each node's flags and old
+// velocity).
+template <int MINB>
+__global__ void __launch_bounds__(G2P_THREADS, MINB) k_g2p(Dev d, Pass p, slosh_particle_t* __restrict__ particles, uint32_t n,
+                                                     const float* __restrict__ vel, const float* __restrict__ disp,
+                                                     uint32_t apply_density) {
+    const uint32_t i = blockIdx.x * G2P_THREADS + threadIdx.x;
+    uint32_t brick = NO_BRICK;
+    uint32_t speed_bits = 0u;
+    if (i < n) {
+        const float4 ra = __ldg(reinterpret_cast<const float4*>(particles + i));
+        if (!is_dead_age(ra.w)) g2p_particle(d, p, particles, i, ra, GlobalField{vel, disp}, apply_density != 0u, brick, speed_bits);
+    }
+    g2p_finish(d, brick, speed_bits);
+}
+
+// APIC: the CTA copies the velocity (and displacement) nodes of its particles' cell box and G2P_MARGIN cells around it into
+// shared memory, where a stencil is one address and seven constant or uniform offsets: the brick pool's form reads the
+// brick table and forms eight indices for each of a particle's six (with the displacement nine) stencils, 1,061 warp
+// instructions per 32 particles without it, 1,430 with it. The margin holds the stencils of the RK2 midpoint up to a step
+// of two cells; positions that leave the tile, and CTAs whose box does not fit, read the pool.
+// Bound by issue (about 60 %) and the phases' latency (box, fill, advect), so CTAs of 384 threads, three per SM at 64
+// registers: 20.6 M particles at 256^3 with the displacement 1,266 us from the pool, 909 now; 6.2 M in 256x128x128 455 and 346;
+// 1.7 M in 128x128x96 101 and 82. 512 threads, two per SM: 1,021; 256, four: 967; 384, four (40 registers): 958. Only positions
+// and ages are read of the records (the old velocity is FLIP's).
+constexpr int G2P_TILE_THREADS = 384;
+constexpr int G2P_MARGIN = 2;
+template <bool DENSITY>
+__global__ void __launch_bounds__(G2P_TILE_THREADS, 3) k_g2p_tile(Dev d, Pass p, slosh_particle_t* __restrict__ particles, uint32_t n,
+                                                                  const float* __restrict__ vel, const float* __restrict__ disp) {
+    extern __shared__ float g2p_tile[];  // [3 or 6][G2P_TILE_NODES]
+    __shared__ int s_box[6];
+    const uint32_t i = blockIdx.x * G2P_TILE_THREADS + threadIdx.x;
+    const int big = 0x7FFFFFFF;
+    if (threadIdx.x < 3) { s_box[threadIdx.x] = big; s_box[3 + threadIdx.x] = -big; }
+    __syncthreads();
+    const float4 ra = i < n ? __ldg(reinterpret_cast<const float4*>(particles + i)) : make_float4(0.0f, 0.0f, 0.0f, -1.0f);
+    const bool live = !is_dead_age(ra.w);
+    int3 mn = make_int3(big, big, big), mx = make_int3(-big, -big, -big);
+    if (live) mn = mx = p2g_cell(d, make_float3(ra.x, ra.y, ra.z));
+    mn.x = __reduce_min_sync(0xFFFFFFFFu, mn.x); mn.y = __reduce_min_sync(0xFFFFFFFFu, mn.y); mn.z = __reduce_min_sync(0xFFFFFFFFu, mn.z);
+    mx.x = __reduce_max_sync(0xFFFFFFFFu, mx.x); mx.y = __reduce_max_sync(0xFFFFFFFFu, mx.y); mx.z = __reduce_max_sync(0xFFFFFFFFu, mx.z);
+    if ((threadIdx.x & 31) == 0 && mn.x <= mx.x) {
+        atomicMin(s_box + 0, mn.x); atomicMin(s_box + 1, mn.y); atomicMin(s_box + 2, mn.z);
+        atomicMax(s_box + 3, mx.x); atomicMax(s_box + 4, mx.y); atomicMax(s_box + 5, mx.z);
+    }
+    __syncthreads();
+    if (s_box[0] == big) return;  // no live particle in this CTA (uniform)
+    TileField F;
+    F.global = GlobalField{vel, disp};
+    F.origin = make_int3(max(s_box[0] - G2P_MARGIN, 0), max(s_box[1] - G2P_MARGIN, 0), max(s_box[2] - G2P_MARGIN, 0));
+    F.dim = make_int3(min(s_box[3] + G2P_MARGIN, d.grid.x - 1) - F.origin.x + 1, min(s_box[4] + G2P_MARGIN, d.grid.y - 1) - F.origin.y + 1,
+                      min(s_box[5] + G2P_MARGIN, d.grid.z - 1) - F.origin.z + 1);
+    F.sy = F.dim.x;
+    F.sz = F.dim.x * F.dim.y;
+    const bool fits = (long long)F.sz * F.dim.z <= G2P_TILE_NODES;
+    F.tile = fits ? g2p_tile : nullptr;
+    if (fits) {
+        const int nodes = F.sz * F.dim.z;
+        // l / sy == __umulhi(l, my) for l, sy < 2^16, sy >= 2 (a grid has at least 4 cells an axis)
+        const uint32_t my = 0xFFFFFFFFu / uint32_t(F.sy) + 1u, mz = 0xFFFFFFFFu / uint32_t(F.sz) + 1u;
+        for (int l = int(threadIdx.x); l < nodes; l += G2P_TILE_THREADS) {
+            const uint32_t lz = __umulhi(uint32_t(l), mz), r = uint32_t(l) - lz * uint32_t(F.sz), ly = __umulhi(r, my), lx = r - ly * uint32_t(F.sy);
+            const int3 c = make_int3(F.origin.x + int(lx), F.origin.y + int(ly), F.origin.z + int(lz));
+            const uint32_t ci = __ldg(d.brick_table + brick_index_of(d, make_int3(c.x >> 3, c.y >> 3, c.z >> 3))) * BRICK_CELLS + local_index_of(c);
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                g2p_tile[a * G2P_TILE_NODES + l] = vel[uint32_t(a) * d.pool_cells + ci];
+                if (DENSITY) g2p_tile[(3 + a) * G2P_TILE_NODES + l] = disp[uint32_t(a) * d.pool_cells + ci];
+            }
+        }
+        __syncthreads();
+    }
+    uint32_t brick = NO_BRICK, speed_bits = 0u;
+    if (live) g2p_particle(d, p, particles, i, ra, F, DENSITY, brick, speed_bits);
+    g2p_finish(d, brick, speed_bits);
 }
 
 }  // namespace
@@ -929,6 +1101,12 @@ int launch_p2g_gather(const Dev& d, const Pass& p, const P2GGather& g, const slo
 int launch_g2p(const Dev& d, const Pass& p, slosh_particle_t* particles, uint32_t n, const float* vel, const float* disp,
                bool apply_density, cudaStream_t s) {
     if (n == 0) return 0;
+    if (p.use_apic) {
+        const int smem = (apply_density ? 6 : 3) * G2P_TILE_NODES * 4;
+        auto kernel = apply_density ? k_g2p_tile<true> : k_g2p_tile<false>;
+        kernel<<<(n + G2P_TILE_THREADS - 1u) / G2P_TILE_THREADS, G2P_TILE_THREADS, smem, s>>>(d, p, particles, n, vel, disp);
+        return 1;
+    }
     // 4 CTAs per SM (64 registers): 5 (48 registers, spills) measured the same, 3 (no spills) 11 % and 2 42 % slower
     k_g2p<4><<<(n + G2P_THREADS - 1u) / G2P_THREADS, G2P_THREADS, 0, s>>>(d, p, particles, n, vel, disp, apply_density ? 1u : 0u);
     return 1;
