@@ -172,7 +172,7 @@ struct Ctx {
     SortBuffers sortb{};
     P2GGather gather{};  // the per-cell particle index of the gather P2G (allocated only when it is on)
     MGState mg{};
-    uint32_t cluster_sizes = 0;    // cluster sizes of the solve's cluster form for this layout (0: not available)
+    int cluster_most = 0;          // most CTAs of the solve's cluster form for this layout (0: not available)
     uint32_t bricks_estimate = 0;  // active bricks of the last frame; the layout's most before the first
 
     // pinned host staging
@@ -456,7 +456,7 @@ struct Ctx {
         total_emitted = 0;
         prev_dt = 0.0f;
         last_max_speed = 0.0f;
-        cluster_sizes = mg_solve_clusters(mg);
+        cluster_most = mg_solve_clusters(mg);
         bricks_estimate = num_pool_bricks - 1u;
         shape.num_sms = num_sms;
         shape.brick_ctas = brick_ctas_for(ctas_per_sm);
@@ -714,7 +714,7 @@ struct Ctx {
         const Dev d = dev();
         // few active bricks: the whole solve in one cluster (the form does not change the result, so the last frame's
         // count, which the host has, is enough to choose by)
-        const int cluster = mg_solve_cluster(cluster_sizes, bricks_estimate);
+        const int cluster = mg_solve_cluster(cluster_most, bricks_estimate);
         SolveGraph* G = nullptr;
         if (use_graphs && cluster == 0) {
             try {

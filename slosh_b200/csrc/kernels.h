@@ -150,11 +150,11 @@ int launch_pcg_init(const Dev& d, const MGState& m, const float* p, const float*
 // solves), then one launch per colour sweep.
 int launch_rbgs_words(const Dev& d, const MGState& m, const Shape& sh, cudaStream_t s);
 int launch_rbgs(const Dev& d, const MGState& m, float* pres, const float* rhs, uint32_t parity, float omega, const Shape& sh, cudaStream_t s);
-// A whole solve (setup and all iterations) as one thread-block cluster, for tanks of few active bricks: the cluster sizes
+// A whole solve (setup and all iterations) as one thread-block cluster, for tanks of few active bricks: the largest cluster
 // a hierarchy can use (this also sets the kernels' attributes on the device), the CTAs for a tank of about `bricks` active
 // bricks (0: use the launched form), and the launch.
-uint32_t mg_solve_clusters(const MGState& m);
-int mg_solve_cluster(uint32_t sizes, uint32_t bricks);
+int mg_solve_clusters(const MGState& m);
+int mg_solve_cluster(int largest, uint32_t bricks);
 int launch_solve_cluster(const Dev& d, const MGState& m, int ctas, float* p, const float* div, uint32_t limit, bool tol_mode, double tol,
                          int coarse, bool setup, cudaStream_t s);
 int launch_vcycle(const Dev& d, const MGState& m, int coarse_iterations, const Shape& sh, cudaStream_t s);

@@ -2279,38 +2279,35 @@ int mid_level(const MGState& m, int tail) {
     return ok ? from : 0;
 }
 
-// The cluster sizes that the solve of this hierarchy can run with on the current device: bit c for a cluster of c CTAs (4
-// to 16, even). 0: none (a single level, an alternative form asked for by the environment, no room).
-uint32_t mg_solve_clusters(const MGState& m) {
-    if (m.num_levels < 2 || mg_staged() || mid_level(m, mg_tail_level(m)) > 0) return 0u;
+// The largest cluster that the solve of this hierarchy can run with on the current device: 16 CTAs, or 8 where no 16 can be
+// placed together, or 0 (a single level, an alternative form asked for by the environment, no room). Smaller clusters of
+// the same CTAs fit wherever a larger one does. (An occupancy query takes milliseconds, so one kernel and size is asked.)
+int mg_solve_clusters(const MGState& m) {
+    if (m.num_levels < 2 || mg_staged() || mid_level(m, mg_tail_level(m)) > 0) return 0;
     const size_t smem = cl_smem(m);
-    if (smem > size_t(CL_MAX_SMEM)) return 0u;
-    uint32_t sizes = 0u;
-    for (int ctas = 4; ctas <= 16; ctas += 2) {
-        bool ok = true;
-        for (int flex = 0; flex < 2 && ok; ++flex) {
-            auto kernel = flex ? k_solve_cluster<true> : k_solve_cluster<false>;
-            cudaLaunchConfig_t cfg = {};
-            cudaLaunchAttribute attr[1];
-            cl_config(cfg, attr, ctas, smem, nullptr);
-            int clusters = 0;
-            ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-                 cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CL_MAX_SMEM) == cudaSuccess &&
-                 cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters > 0;
-        }
-        cudaGetLastError();
-        if (ok) sizes |= 1u << ctas;
+    if (smem > size_t(CL_MAX_SMEM)) return 0;
+    bool ok = true;
+    for (auto kernel : {k_solve_cluster<false>, k_solve_cluster<true>})
+        ok = ok && cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+             cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CL_MAX_SMEM) == cudaSuccess;
+    for (int ctas : {16, 8}) {
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr[1];
+        cl_config(cfg, attr, ctas, smem, nullptr);
+        int clusters = 0;
+        if (ok && cudaOccupancyMaxActiveClusters(&clusters, k_solve_cluster<true>, &cfg) == cudaSuccess && clusters > 0) return ctas;
     }
-    return sizes;
+    cudaGetLastError();
+    return 0;
 }
 // The cluster for a tank of about `bricks` active bricks: the smallest whose resident form holds them with a sixteenth to
 // spare, so that several tanks' clusters fit the GPU at once (a solve's passes take as long on few SMs as on many while
 // each warp has one brick). 0, the launched form, for tanks that no cluster holds: the streamed form, which takes over
 // when a tank outgrows its cluster within a frame, is slower than launches over the whole GPU (64^3, 240 to 300 active
 // bricks: 1.8 against 1.3 ms a frame).
-int mg_solve_cluster(uint32_t sizes, uint32_t bricks) {
-    for (int ctas = 4; ctas <= 16; ctas += 2)
-        if (((sizes >> ctas) & 1u) && bricks + bricks / 16u <= uint32_t(ctas - 1) * uint32_t(CL_WARPS)) return ctas;
+int mg_solve_cluster(int largest, uint32_t bricks) {
+    for (int ctas = 4; ctas <= largest; ctas += 2)
+        if (bricks + bricks / 16u <= uint32_t(ctas - 1) * uint32_t(CL_WARPS)) return ctas;
     return 0;
 }
 int launch_solve_cluster(const Dev& d, const MGState& m, int ctas, float* p, const float* div, uint32_t limit, bool tol_mode, double tol,
