@@ -438,7 +438,14 @@ struct Ctx {
         {
             size_t tail_cells = 0;
             for (int l = 1; l < num_levels; ++l) tail_cells += level_cells[l];
+            const int tail = mg_tail_level(mg);
             mg.tail_list = dalloc<uint32_t>(tail_cells + 1, false);
+            // the lists take the words of the tail's levels; the levels above them keep their x2 in the rest
+            size_t used = 1;
+            for (int l = num_levels - 1; l >= 1; --l) {
+                mg.lv[l].x2 = l < tail ? reinterpret_cast<float*>(mg.tail_list + used) : nullptr;
+                used += level_cells[l];
+            }
             mg.tail_meta = dalloc<uint32_t>(4 * SLOSH_MAX_MG_LEVELS, false);
             mg.tail_image = dalloc<unsigned char>(mg_tail_smem(mg) + 16, false);
         }

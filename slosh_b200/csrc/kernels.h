@@ -107,6 +107,7 @@ struct MGLevel {
     uint32_t cells;
     uint32_t* type;
     float* x;
+    float* x2;        // levels 1 to the tail: x between the descent and the ascent of the fused passes
     float* b;
     uint16_t* word;   // per-solve stencil word: bits 0-5 fluid neighbour, 6 fluid, 7 red, 8-13 non-solid neighbour
     uint32_t prec;    // storage of x and b: SLOSH_PRECISION_FP32, _FP16_STORAGE (2-byte halves) or _BF16_STORAGE

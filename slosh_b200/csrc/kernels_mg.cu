@@ -1040,6 +1040,183 @@ __global__ void k_prolong_smooth_fp(Dev d, MGState m, int l) {
     else for_footprint(d, F, l, [&](uint32_t i, int3 c) { prolong_smooth_fp_cell(F, C, i, c); });
 }
 
+// ---- a coarse level's whole descent or ascent in one pass -------------------------------------------------------
+// A level's smoothing is 2 S colour sweeps, of which each cell's value depends on cells at most that many steps away, so a
+// CTA that loads an 8^3 tile of the level with a halo of 2 S cells can run all of them (and the restriction behind, or the
+// prolongation before) in shared memory, computing the halo's cells again where its neighbours compute them too: the same
+// operations on the same values, so the same bits. One launch instead of 2 S for the descent and 2 S for the ascent, each of
+// which took 4-7 us for a few thousand cells. The descent reads x (the restriction's red initialisation) from the level's x
+// and writes x2, the ascent reads x2 and writes x, so no CTA reads what another writes.
+// Cells outside the active bricks' footprints keep the words of an earlier solve; what is computed for them is read by none
+// (the fresh words' fluid-neighbour bits never point at them, and their parents are air).
+// Bound by the passes' chain (tile test, loads, sweeps) and by the halo's work, three times the tile's own for S = 2. CTAs of
+// 1,024 threads: pressure of a 256^3 substep (fused from level 2) 2,257 -> 2,183 us, of the 256x128x128 boxes (from level 1,
+// 1,024 tiles) 1,876 -> 1,608, of 128x128x96 substeps with one sweep pair (from level 2) 815 -> 784 a frame. With 256 threads and
+// 4 loads in flight slower than the launches (2,603 us); level 1 of 256^3 (4,096 tiles, most of them empty) too (2,567 us, 2,297
+// with a list of the tiles that hold active bricks).
+constexpr int CT_SIDE = 8, CT_THREADS = 1024, CT_LEVEL1_TILES = 1536;
+template <int S> struct CoarseTile {
+    static constexpr int H = 2 * S, R = CT_SIDE + 2 * H, CELLS = R * R * R;
+    float x[CELLS], b[CELLS];
+    uint16_t w[CELLS];
+    float res[CT_SIDE * CT_SIDE * CT_SIDE];
+    float dt[16];  // diagonal and its reciprocal by count of non-solid neighbours
+};
+__device__ __forceinline__ uint32_t word_nonsolid(uint32_t w) { return uint32_t(__popc((w >> CW_NONSOLID_SHIFT) & 63u)); }
+template <int S>
+__device__ __forceinline__ float ct_sum(const CoarseTile<S>& T, uint32_t w, int i) {
+    constexpr int R = CoarseTile<S>::R;
+    const int off[6] = {i - 1, i + 1, i - R, i + R, i - R * R, i + R * R};
+    float v[6], sum = 0.0f;
+#pragma unroll
+    for (int n = 0; n < 6; ++n) v[n] = T.x[off[n]];
+#pragma unroll
+    for (int n = 0; n < 6; ++n)
+        if ((w >> n) & 1u) sum = sum + v[n];
+    return sum;
+}
+// One colour (parity 0: red) of the cells at most D steps outside the tile.
+template <int S, int D>
+__device__ __forceinline__ void ct_sweep(CoarseTile<S>& T, uint32_t parity, uint32_t prec) {
+    constexpr int R = CoarseTile<S>::R, H = CoarseTile<S>::H, N = CT_SIDE + 2 * D;
+    static_assert(N <= 16, "a z plane's cells of a colour fit 128 threads");
+    // threads 8 (half row) x 16 (row) x CT_THREADS / 128 (planes). Tile origins are even and D shifts all three axes alike,
+    // so a cell's colour is that of its local coordinates.
+    const int xh = int(threadIdx.x & 7u), y = int((threadIdx.x >> 3) & 15u);
+    for (int z = int(threadIdx.x >> 7); z < N; z += CT_THREADS / 128) {
+        if (xh >= N / 2 || y >= N) break;
+        const int x = 2 * xh + ((y + z + int(parity) + D) & 1);
+        const int i = (x + H - D) + R * ((y + H - D) + R * (z + H - D));
+        const uint32_t w = T.w[i];
+        if (!(w & CW_FLUID)) continue;
+        const uint32_t c = word_nonsolid(w);
+        T.x[i] = q_prec(div_by(T.b[i] + ct_sum<S>(T, w, i), T.dt[c], T.dt[8u + c]), prec);
+    }
+    __syncthreads();
+}
+// The sweeps that bring the tile from a valid halo of D + 1 cells to one of E, alternating from colour `parity`.
+template <int S, int D, int E>
+__device__ __forceinline__ void ct_sweeps(CoarseTile<S>& T, uint32_t parity, uint32_t prec) {
+    if constexpr (D >= E) {
+        ct_sweep<S, D>(T, parity, prec);
+        ct_sweeps<S, D - 1, E>(T, parity ^ 1u, prec);
+    }
+}
+// Loads the tile at o; false (uniformly) when its own cells hold no fluid. value(i, c): x of cell c (index i in L).
+template <int S, class Value>
+__device__ __forceinline__ bool ct_load(CoarseTile<S>& T, const MGLevel& L, int3 o, Value value) {
+    constexpr int R = CoarseTile<S>::R, H = CoarseTile<S>::H;
+    if (threadIdx.x < 7u) {
+        T.dt[threadIdx.x] = word_diag(((1u << threadIdx.x) - 1u) << CW_NONSOLID_SHIFT);
+        T.dt[8u + threadIdx.x] = 1.0f / T.dt[threadIdx.x];
+    }
+    bool fluid = false;
+    if (threadIdx.x < uint32_t(CT_SIDE * CT_SIDE * CT_SIDE)) {
+        const int3 c = make_int3(o.x + int(threadIdx.x & 7u), o.y + int((threadIdx.x >> 3) & 7u), o.z + int(threadIdx.x >> 6));
+        fluid = inside3(c, L.dim) && (L.word[lin3(c, L.dim)] & CW_FLUID) != 0u;
+    }
+    if (!__syncthreads_or(fluid)) return false;
+    constexpr int PER = (CoarseTile<S>::CELLS + CT_THREADS - 1) / CT_THREADS, B = PER < 8 ? PER : 8;
+    for (int k0 = 0; k0 < PER; k0 += B) {  // B cells' loads in flight: indices are clamped into the level, outside it the word is 0
+        uint32_t w[B];
+        float x[B], b[B];
+#pragma unroll
+        for (int k = 0; k < B; ++k) {
+            const int i = int(threadIdx.x) + (k0 + k) * CT_THREADS;
+            const int3 c = make_int3(o.x - H + i % R, o.y - H + (i / R) % R, o.z - H + i / (R * R));
+            const int3 q = make_int3(min(max(c.x, 0), L.dim.x - 1), min(max(c.y, 0), L.dim.y - 1), min(max(c.z, 0), L.dim.z - 1));
+            const uint32_t ci = lin3(q, L.dim);
+            w[k] = inside3(c, L.dim) ? uint32_t(L.word[ci]) : 0u;
+            x[k] = value(ci, q);
+            b[k] = lv_ld(L.b, ci, L.prec);
+        }
+#pragma unroll
+        for (int k = 0; k < B; ++k) {
+            const int i = int(threadIdx.x) + (k0 + k) * CT_THREADS;
+            if (i >= CoarseTile<S>::CELLS) break;
+            T.w[i] = uint16_t(w[k]);
+            T.x[i] = x[k];
+            T.b[i] = b[k];
+        }
+    }
+    __syncthreads();
+    return true;
+}
+template <int S>
+__device__ __forceinline__ void ct_store(const CoarseTile<S>& T, const MGLevel& L, int3 o, float* out) {
+    constexpr int R = CoarseTile<S>::R, H = CoarseTile<S>::H;
+    for (uint32_t j = threadIdx.x; j < uint32_t(CT_SIDE * CT_SIDE * CT_SIDE); j += CT_THREADS) {
+        const int x = int(j & 7u), y = int((j >> 3) & 7u), z = int(j >> 6), i = (x + H) + R * ((y + H) + R * (z + H));
+        if (T.w[i] & CW_FLUID) lv_st(out, lin3(make_int3(o.x + x, o.y + y, o.z + z), L.dim), L.prec, T.x[i]);
+    }
+}
+__host__ __device__ __forceinline__ int3 ct_tiles(const MGLevel& L) {
+    return make_int3((L.dim.x + CT_SIDE - 1) / CT_SIDE, (L.dim.y + CT_SIDE - 1) / CT_SIDE, (L.dim.z + CT_SIDE - 1) / CT_SIDE);
+}
+__device__ __forceinline__ int3 ct_origin(const MGLevel& L) {
+    const int3 n = ct_tiles(L);
+    const uint32_t t = blockIdx.x;
+    return make_int3(int(t % uint32_t(n.x)) * CT_SIDE, int((t / uint32_t(n.x)) % uint32_t(n.y)) * CT_SIDE, int(t / uint32_t(n.x * n.y)) * CT_SIDE);
+}
+// Pre-smoothing of level l (black, then S - 1 red-black pairs) and its restriction to level l + 1.
+template <int S>
+__global__ void __launch_bounds__(CT_THREADS) k_coarse_down(MGState m, int l) {
+    pdl_entry();
+    __shared__ CoarseTile<S> T;
+    constexpr int R = CoarseTile<S>::R, H = CoarseTile<S>::H;
+    const MGLevel L = m.lv[l], C = m.lv[l + 1];
+    const int3 o = ct_origin(L);
+    const bool fluid = ct_load<S>(T, L, o, [&](uint32_t ci, int3) { return lv_ld(L.x, ci, L.prec); });
+    if (fluid) {
+        ct_sweeps<S, 2 * S - 1, 1>(T, 1u, L.prec);
+        ct_store<S>(T, L, o, L.x2);
+        for (uint32_t j = threadIdx.x; j < uint32_t(CT_SIDE * CT_SIDE * CT_SIDE); j += CT_THREADS) {
+            const int i = (int(j & 7u) + H) + R * ((int((j >> 3) & 7u) + H) + R * (int(j >> 6) + H));
+            const uint32_t w = T.w[i];
+            T.res[j] = T.b[i] - (T.dt[word_nonsolid(w)] * T.x[i] - ct_sum<S>(T, w, i));
+        }
+        __syncthreads();
+    }
+    // a tile without fluid still clears its coarse cells, as the launched pass does
+    if (threadIdx.x < 64u) {
+        const int x = int(threadIdx.x & 3u), y = int((threadIdx.x >> 2) & 3u), z = int(threadIdx.x >> 4);
+        const int3 c = make_int3(o.x / 2 + x, o.y / 2 + y, o.z / 2 + z);
+        if (inside3(c, C.dim)) {
+            const uint32_t ci = lin3(c, C.dim), cw = C.word[ci];
+            float bb = 0.0f, xx = 0.0f;
+            if (fluid && (cw & CW_FLUID)) {
+                float sum = 0.0f;
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    const int fx = 2 * x + (k & 1), fy = 2 * y + ((k >> 1) & 1), fz = 2 * z + (k >> 2);
+                    if (T.w[(fx + H) + R * ((fy + H) + R * (fz + H))] & CW_FLUID) sum = sum + T.res[fx + 8 * (fy + 8 * fz)];
+                }
+                bb = m.restrict_scale * sum;
+                const uint32_t n = word_nonsolid(cw);
+                xx = (cw & CW_RED) ? div_by(bb, T.dt[n], T.dt[8u + n]) : 0.0f;
+            }
+            lv_st(C.b, ci, C.prec, bb);
+            lv_st(C.x, ci, C.prec, xx);
+        }
+    }
+}
+// Prolongation from level l + 1 and post-smoothing of level l (S black-red pairs).
+template <int S>
+__global__ void __launch_bounds__(CT_THREADS) k_coarse_up(MGState m, int l) {
+    pdl_entry();
+    __shared__ CoarseTile<S> T;
+    const MGLevel L = m.lv[l], C = m.lv[l + 1];
+    const int3 o = ct_origin(L);
+    if (!ct_load<S>(T, L, o, [&](uint32_t ci, int3 c) {
+            const uint32_t pi = lin3(make_int3(c.x / 2, c.y / 2, c.z / 2), C.dim);
+            const float x = lv_ld(L.x2, ci, L.prec), px = lv_ld(C.x, pi, C.prec);
+            return (C.word[pi] & CW_FLUID) ? q_prec(x + px, L.prec) : x;
+        }))
+        return;
+    ct_sweeps<S, 2 * S - 1, 0>(T, 1u, L.prec);
+    ct_store<S>(T, L, o, L.x);
+}
+
 // ---- MGRestrictCS level 0 -> 1 over the 4^3 level-1 cells of every active brick (SparseCoarse) -----------
 // One warp per brick: the lanes form the fine residuals of the brick's 512 cells in warp-private shared
 // memory, then sum each of the 64 coarse cells' fluid children in child order (x fastest), as the
@@ -1712,7 +1889,6 @@ struct SLevel {
     uint32_t nred, nblack;
     uint32_t prec;         // storage precision: stores round to it (the values stay FP32 in shared memory)
 };
-__device__ __forceinline__ uint32_t word_nonsolid(uint32_t w) { return uint32_t(__popc((w >> CW_NONSOLID_SHIFT) & 63u)); }
 __device__ __forceinline__ void s_sweep(const SLevel L, uint32_t colour) {
     const uint32_t n = colour == 0u ? L.nred : L.nblack;
     const uint32_t* list = L.list + (colour == 0u ? 0u : L.nred);
@@ -2443,7 +2619,20 @@ int launch_vcycle(const Dev& d, const MGState& m, int coarse_iterations, const S
     }
     const int mid = mid_level(m, tail);  // levels mid..tail-1 and the tail in one cluster (0: separate passes)
     const int down_end = mid > 0 ? mid - 1 : tail;
+    auto tiles = [&](int l) {
+        const int3 t = ct_tiles(m.lv[l]);
+        return t.x * t.y * t.z;
+    };
+    // levels from here to the tail run one fused pass each way: level 2 up, and level 1 where two sweep pairs leave it the
+    // most launches and its tiles are few (mostly empty tiles and the halo's work cost more than launches beyond that)
+    const int fused = mid > 0 || sweeps > 2 ? tail : (sweeps == 2 && tiles(1) <= CT_LEVEL1_TILES ? 1 : 2);
     for (int l = 0; l < down_end; ++l) {
+        if (l >= fused) {
+            if (sweeps == 1) launch_k(k_coarse_down<1>, tiles(l), CT_THREADS, 0, s, m, l);
+            else launch_k(k_coarse_down<2>, tiles(l), CT_THREADS, 0, s, m, l);
+            ++n;
+            continue;
+        }
         if (l == 0) {
             if (staged) ST_LAUNCH(k_restrict0_st, 1, 2, d, m, sh, s);
             else launch_k(k_restrict0, sh.mg_ctas, GRID_THREADS, 0, s, d, m);
@@ -2451,7 +2640,7 @@ int launch_vcycle(const Dev& d, const MGState& m, int coarse_iterations, const S
             launch_k(k_restrict_fp, fp_blocks(l + 1), 256, 0, s, d, m, l);
         }
         ++n;
-        if (l + 1 < tail) {  // the tail kernel does its own pre-smoothing
+        if (l + 1 < std::min(tail, fused)) {  // the tail kernel and the fused passes do their own pre-smoothing
             launch_k(k_smooth_fp, fp_blocks_sweep(l + 1), 256, 0, s, d, m, l + 1, 1u);
             ++n;
             for (int k = 1; k < sweeps; ++k) {
@@ -2480,6 +2669,12 @@ int launch_vcycle(const Dev& d, const MGState& m, int coarse_iterations, const S
     }
     ++n;
     for (int l = (mid > 0 ? mid - 1 : tail - 1); l >= 0; --l) {
+        if (l >= fused) {
+            if (sweeps == 1) launch_k(k_coarse_up<1>, tiles(l), CT_THREADS, 0, s, m, l);
+            else launch_k(k_coarse_up<2>, tiles(l), CT_THREADS, 0, s, m, l);
+            ++n;
+            continue;
+        }
         if (l == 0) {
             if (staged) ST_LAUNCH(k_prolong_smooth0_st, 1, 2, d, m, sh, s);
             else launch_k(k_prolong_smooth0, sh.mg_ctas, GRID_THREADS, 0, s, d, m);
