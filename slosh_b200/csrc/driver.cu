@@ -854,11 +854,13 @@ struct Ctx {
             count(launch_mark_cells(d, P, shape, stream));
             count(launch_normalize_faces(d, P, V[0], shape, stream));
             if (P.viscosity_alpha > 0.0f && S.viscosity_iterations > 0) {
-                CK(cudaMemcpyAsync(V[1], V[0], size_t(total_faces) * 4, cudaMemcpyDeviceToDevice, stream));
+                // the words lie in the solver's q, which no solve uses now; the first iteration's source is the field itself
+                uint8_t* words = reinterpret_cast<uint8_t*>(mg.q);
+                count(launch_viscosity_words(d, words, shape, stream));
                 int src = 1;
                 for (int it = 0; it < S.viscosity_iterations; ++it) {
                     const int dst = src == 1 ? 2 : 1;
-                    count(launch_viscosity(d, P, V[0], V[src], V[dst], shape, stream));
+                    count(launch_viscosity(d, P, words, V[0], V[it == 0 ? 0 : src], V[dst], shape, stream));
                     src = dst;
                 }
                 c = src;
@@ -877,7 +879,7 @@ struct Ctx {
                 const float omega = clampf_h(S.sor_weight, 0.5f, 1.95f);
                 count(launch_rbgs_words(d, mg, shape, stream));
                 for (int it = 0; it < S.pressure_iterations; ++it)
-                    for (uint32_t colour = 0; colour < 2u; ++colour) count(launch_rbgs(d, mg, pressure, divergence, colour, omega, shape, stream));
+                    for (uint32_t colour = 0; colour < 2u; ++colour) count(launch_rbgs(d, mg, pressure, divergence, colour, omega, bricks_estimate, shape, stream));
                 last_iterations = S.pressure_iterations;
                 last_converged = true;
             }
@@ -898,7 +900,7 @@ struct Ctx {
             } else {
                 for (int it = 0; it < std::max(S.density_projection_iterations, 1); ++it)
                     for (uint32_t colour = 0; colour < 2u; ++colour)
-                        count(launch_rbgs(d, mg, density_q, density_rhs, colour, 1.7f, shape, stream));
+                        count(launch_rbgs(d, mg, density_q, density_rhs, colour, 1.7f, bricks_estimate, shape, stream));
             }
         }
         {

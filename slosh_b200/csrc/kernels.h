@@ -45,7 +45,10 @@ int launch_clear_new_slots(const Dev& d, const Shape& sh, cudaStream_t s);
 // ---- grid passes ----
 int launch_mark_cells(const Dev& d, const Pass& p, const Shape& sh, cudaStream_t s);
 int launch_normalize_faces(const Dev& d, const Pass& p, float* vel, const Shape& sh, cudaStream_t s);
-int launch_viscosity(const Dev& d, const Pass& p, const float* ustar, const float* src, float* dst, const Shape& sh, cudaStream_t s);
+// One Jacobi iteration of the viscosity; words: 3 x pool_cells bytes, built once per substep from the face flags.
+int launch_viscosity_words(const Dev& d, uint8_t* words, const Shape& sh, cudaStream_t s);
+int launch_viscosity(const Dev& d, const Pass& p, const uint8_t* words, const float* ustar, const float* src, float* dst, const Shape& sh,
+                     cudaStream_t s);
 int launch_divergence(const Dev& d, const Pass& p, const float* vel, const Shape& sh, cudaStream_t s);
 int launch_project(const Dev& d, const Pass& p, float* vel, const Shape& sh, cudaStream_t s);
 int launch_residual(const Dev& d, const Pass& p, const float* vel, const Shape& sh, cudaStream_t s);
@@ -150,7 +153,9 @@ int launch_pcg_init(const Dev& d, const MGState& m, const float* p, const float*
 // Red-black SOR (PressureRBGSCS): the stencil words and neighbour slots of this substep's cell types (once for both its
 // solves), then one launch per colour sweep.
 int launch_rbgs_words(const Dev& d, const MGState& m, const Shape& sh, cudaStream_t s);
-int launch_rbgs(const Dev& d, const MGState& m, float* pres, const float* rhs, uint32_t parity, float omega, const Shape& sh, cudaStream_t s);
+// bricks: about how many are active (chooses the split of a brick over warps, not the result).
+int launch_rbgs(const Dev& d, const MGState& m, float* pres, const float* rhs, uint32_t parity, float omega, uint32_t bricks, const Shape& sh,
+                cudaStream_t s);
 // A whole solve (setup and all iterations) as one thread-block cluster, for tanks of few active bricks: the largest cluster
 // a hierarchy can use (this also sets the kernels' attributes on the device), the CTAs for a tank of about `bricks` active
 // bricks (0: use the launched form), and the launch.

@@ -426,24 +426,29 @@ __device__ __forceinline__ void w0_black(const Dev& d, const MGState& m, Prep pr
 // the brick table and the neighbour's type before each value. A colour's cells are read by other warps only through
 // the other colour's sweep, so reading and writing one array is safe.
 // Bound by L2 latency and bandwidth: 192^3 with 1.09 M fluid cells 23.3 us a colour before, 5.9 now (a frame of 200 + 30
-// iterations 11.8 -> 3.6 ms); 96x96x72 with 0.1 M fluid cells 8.8 -> 4.8 us. Half a brick per warp (one round of loads)
-// takes 1.25 instead of 1.41 ms for a frame of the small tank but 4.0 instead of 3.6 ms for the large one.
+// iterations 11.8 -> 3.6 ms); 96x96x72 with 0.1 M fluid cells 8.8 -> 4.8 us. PARTS = 2: half a brick per warp, one round of loads
+// instead of two, while all of the halves are resident (RB_HALF_BRICKS): a frame of the small tank 1.41 -> 1.25 ms; the large
+// one takes 4.0 instead of 3.6 ms so.
+constexpr uint32_t RB_HALF_BRICKS = 1500;
 __device__ __forceinline__ uint32_t colour_local(uint32_t lane, uint32_t k, uint32_t parity) {
     const uint32_t y = lane >> 2;
     return 2u * (lane & 3u) + ((y + k + parity) & 1u) + 8u * y + 64u * k;
 }
+template <uint32_t PARTS>
 __global__ void __launch_bounds__(GRID_THREADS) k_rbgs(Dev d, MGState m, float* pres, const float* __restrict__ rhs, uint32_t parity, float omega) {
     pdl_entry();
     constexpr uint32_t B = 4u;
-    const uint32_t active = d.active_bricks[0];
+    const uint32_t active = PARTS * d.active_bricks[0];
     const uint32_t lane = threadIdx.x & 31u, wpb = blockDim.x >> 5;
-    for (uint32_t e = blockIdx.x * wpb + (threadIdx.x >> 5); e < active; e += gridDim.x * wpb) {
+    for (uint32_t t = blockIdx.x * wpb + (threadIdx.x >> 5); t < active; t += gridDim.x * wpb) {
+        const uint32_t e = t / PARTS, first = (8u / PARTS) * (t % PARTS);
         const uint4 s0 = *reinterpret_cast<const uint4*>(m.nbr_slots + 8u * e);
         const uint4 s1 = *reinterpret_cast<const uint4*>(m.nbr_slots + 8u * e + 4u);
         const uint32_t ns[6] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y};
         const uint32_t base = s1.z * BRICK_CELLS;
 #pragma unroll
-        for (uint32_t k0 = 0; k0 < 8u; k0 += B) {
+        for (uint32_t kk = 0; kk < 8u / PARTS; kk += B) {
+            const uint32_t k0 = first + kk;
             uint32_t w[B];
             float b[B], dg[B], old[B], n[B][6];
 #pragma unroll
@@ -2701,8 +2706,9 @@ int launch_rbgs_words(const Dev& d, const MGState& m, const Shape& sh, cudaStrea
     launch_k(k_pcg_words, sh.mg_ctas, GRID_THREADS, 0, s, d, m);
     return 1;
 }
-int launch_rbgs(const Dev& d, const MGState& m, float* pres, const float* rhs, uint32_t parity, float omega, const Shape& sh, cudaStream_t s) {
-    launch_k(k_rbgs, sh.mg_ctas, GRID_THREADS, 0, s, d, m, pres, rhs, parity, omega);
+int launch_rbgs(const Dev& d, const MGState& m, float* pres, const float* rhs, uint32_t parity, float omega, uint32_t bricks, const Shape& sh,
+                cudaStream_t s) {
+    launch_k(bricks <= RB_HALF_BRICKS ? k_rbgs<2> : k_rbgs<1>, sh.mg_ctas, GRID_THREADS, 0, s, d, m, pres, rhs, parity, omega);
     return 1;
 }
 int launch_pcg_apply_a(const Dev& d, const MGState& m, const Shape& sh, cudaStream_t s) {
