@@ -461,23 +461,33 @@ __global__ void __launch_bounds__(128) k_wgrad(const __grid_constant__ WgradArgs
 }
 
 // out[i] = sum over chunks of partial[chunk][i], in chunk order.
-__global__ void k_reduce_chunks(const float* __restrict__ partial, float* __restrict__ out, uint32_t chunks, uint32_t count) {
+// The sum of a value's chunks in chunk order. The additions are a chain, but BATCH loads are in flight at a time: at most
+// four were before, and 17 weight gradients' sums took 8.0 us each (now 4.4), 14 bias gradients' 7.4.
+template <uint32_t BATCH>
+__device__ __forceinline__ float sum_chunks(const float* __restrict__ p, uint32_t chunks, uint32_t stride) {
+    float s = 0.0f;
+    uint32_t c = 0;
+    for (; c + BATCH <= chunks; c += BATCH) {
+        float v[BATCH];
+#pragma unroll
+        for (uint32_t k = 0; k < BATCH; ++k) v[k] = p[uint64_t(c + k) * stride];
+#pragma unroll
+        for (uint32_t k = 0; k < BATCH; ++k) s = s + v[k];
+    }
+    for (; c < chunks; ++c) s = s + p[uint64_t(c) * stride];
+    return s;
+}
+__global__ void __launch_bounds__(256) k_reduce_chunks(const float* __restrict__ partial, float* __restrict__ out, uint32_t chunks, uint32_t count) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
-    float s = 0.0f;
-    for (uint32_t c = 0; c < chunks; ++c) s = s + partial[uint64_t(c) * count + i];
-    out[i] = s;
+    out[i] = sum_chunks<64>(partial + i, chunks, count);  // few values of many chunks: one round trip per 64
 }
-
-// Weight gradient of one K-block: out[(tap n + co) cin + off + cl] = sum over chunks of
-// partial[chunk][tap][co][cl], in chunk order.
 __global__ void k_reduce_wgrad(const float* __restrict__ partial, float* __restrict__ out, uint32_t chunks, uint32_t n, uint32_t cb,
                                uint32_t cin, uint32_t off) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t count = 27u * n * cb;
     if (i >= count) return;
-    float s = 0.0f;
-    for (uint32_t c = 0; c < chunks; ++c) s = s + partial[uint64_t(c) * count + i];
+    const float s = sum_chunks<16>(partial + i, chunks, count);
     const uint32_t cl = i % cb, row = i / cb;
     out[row * cin + off + cl] = s;
 }
@@ -490,8 +500,17 @@ __global__ void k_bias_partial(const bf16* __restrict__ g, uint32_t n, uint64_t 
     const uint64_t v0 = uint64_t(blockIdx.x) * per_chunk;
     const uint64_t v1 = min(voxels, v0 + per_chunk);
     float s = 0.0f;
-    if (q < lanes)
-        for (uint64_t v = v0 + q; v < v1; v += lanes) s = s + bf(g[v * n + j]);
+    if (q < lanes) {
+        uint64_t v = v0 + q;
+        for (; v + 15u * lanes < v1; v += 16u * lanes) {  // 16 loads in flight, added in order
+            bf16 t[16];
+#pragma unroll
+            for (uint32_t k = 0; k < 16u; ++k) t[k] = g[(v + k * lanes) * n + j];
+#pragma unroll
+            for (uint32_t k = 0; k < 16u; ++k) s = s + bf(t[k]);
+        }
+        for (; v < v1; v += lanes) s = s + bf(g[v * n + j]);
+    }
     s_sum[threadIdx.x] = s;
     __syncthreads();
     if (threadIdx.x < n) {
