@@ -877,9 +877,7 @@ struct Ctx {
                 else mgpcg(pressure, divergence, S.pcg_iterations, 0.0f, 0, coarse, 0);
             } else {
                 const float omega = clampf_h(S.sor_weight, 0.5f, 1.95f);
-                count(launch_rbgs_words(d, mg, shape, stream));
-                for (int it = 0; it < S.pressure_iterations; ++it)
-                    for (uint32_t colour = 0; colour < 2u; ++colour) count(launch_rbgs(d, mg, pressure, divergence, colour, omega, bricks_estimate, shape, stream));
+                count(launch_rbgs(d, mg, pressure, divergence, S.pressure_iterations, omega, true, bricks_estimate, shape, stream));
                 last_iterations = S.pressure_iterations;
                 last_converged = true;
             }
@@ -898,9 +896,7 @@ struct Ctx {
             if (S.pressure_solver == SLOSH_SOLVER_MGPCG) {
                 mgpcg(density_q, density_rhs, 2, 0.0f, 0, clampi_h(S.mg_coarse_iterations, 1, 200), 1);
             } else {
-                for (int it = 0; it < std::max(S.density_projection_iterations, 1); ++it)
-                    for (uint32_t colour = 0; colour < 2u; ++colour)
-                        count(launch_rbgs(d, mg, density_q, density_rhs, colour, 1.7f, bricks_estimate, shape, stream));
+                count(launch_rbgs(d, mg, density_q, density_rhs, std::max(S.density_projection_iterations, 1), 1.7f, false, bricks_estimate, shape, stream));
             }
         }
         {

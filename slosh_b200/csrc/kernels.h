@@ -150,11 +150,11 @@ int launch_mg_coarse_setup(const Dev& d, const MGState& m, const Shape& sh, cuda
 // handle: the WHILE node's condition when the solve runs as a CUDA graph, 0 otherwise.
 int launch_pcg_init(const Dev& d, const MGState& m, const float* p, const float* div, unsigned long long handle, const Shape& sh,
                     cudaStream_t s, bool words = true);
-// Red-black SOR (PressureRBGSCS): the stencil words and neighbour slots of this substep's cell types (once for both its
-// solves), then one launch per colour sweep.
-int launch_rbgs_words(const Dev& d, const MGState& m, const Shape& sh, cudaStream_t s);
-// bricks: about how many are active (chooses the split of a brick over warps, not the result).
-int launch_rbgs(const Dev& d, const MGState& m, float* pres, const float* rhs, uint32_t parity, float omega, uint32_t bricks, const Shape& sh,
+// Red-black SOR (PressureRBGSCS): `sweeps` sweeps over pres, one launch per colour between the split by colour and the merge.
+// first: a substep's first solve, which also makes the stencil words and neighbour slots of its cell types (its second one
+// uses them again; nothing may write m's level-0 arrays in between). bricks: about how many are active (chooses the
+// split of a brick over warps, not the result).
+int launch_rbgs(const Dev& d, const MGState& m, float* pres, const float* rhs, int sweeps, float omega, bool first, uint32_t bricks, const Shape& sh,
                 cudaStream_t s);
 // A whole solve (setup and all iterations) as one thread-block cluster, for tanks of few active bricks: the largest cluster
 // a hierarchy can use (this also sets the kernels' attributes on the device), the CTAs for a tank of about `bricks` active

@@ -420,56 +420,138 @@ __device__ __forceinline__ void w0_black(const Dev& d, const MGState& m, Prep pr
 }
 
 // ---- PressureRBGSCS: one SOR colour sweep ----------------------------------------------------------------
-// Reference: PLUG/Shaders/Private/Slosh.usf:860-892. The cells of one colour (parity 0: red) of every active brick, one
-// warp per brick, 8 cells per lane as in w0_black, with the per-solve stencil words and neighbour slots (k_pcg_words)
-// that the MGPCG passes use: all nine loads of four cells are in flight at once, where the sweep over cell types read
-// the brick table and the neighbour's type before each value. A colour's cells are read by other warps only through
-// the other colour's sweep, so reading and writing one array is safe.
-// Bound by L2 latency and bandwidth: 192^3 with 1.09 M fluid cells 23.3 us a colour before, 5.9 now (a frame of 200 + 30
-// iterations 11.8 -> 3.6 ms); 96x96x72 with 0.1 M fluid cells 8.8 -> 4.8 us. PARTS = 2: half a brick per warp, one round of loads
-// instead of two, while all of the halves are resident (RB_HALF_BRICKS): a frame of the small tank 1.41 -> 1.25 ms; the large
-// one takes 4.0 instead of 3.6 ms so.
-constexpr uint32_t RB_HALF_BRICKS = 1500;
-__device__ __forceinline__ uint32_t colour_local(uint32_t lane, uint32_t k, uint32_t parity) {
-    const uint32_t y = lane >> 2;
-    return 2u * (lane & 3u) + ((y + k + parity) & 1u) + 8u * y + 64u * k;
+// Reference: PLUG/Shaders/Private/Slosh.usf:860-892. A colour's cells are every second one of a row: in cell order a
+// sweep moves every sector of every array and uses half of each. So a solve keeps its arrays by colour, in the MGPCG
+// solve's vectors (which the SOR solver leaves idle): cell (x, y, z) of a brick is entry (x >> 1) + 4 y + 32 z of its
+// colour's 256; the pressure in z, the right-hand side in r, the diagonal in dvec, the stencil words in q (a cell without a
+// diagonal counts as no fluid). k_rbgs_split fills them, k_rbgs sweeps over them and k_rbgs_merge returns the pressure.
+// One warp per active brick, two entries of a row per lane and round: the y and z neighbours and three of the four x
+// neighbours are 8-byte loads of the other colour. A colour's cells are read by other warps only through the other
+// colour's sweep, so reading and writing one array is safe.
+// Bound by L2 latency and bandwidth: 192^3 with 1.09 M fluid cells 23.3 us a colour over cell types, 5.9 over stencil words in
+// cell order, 5.0 so (a frame of 200 + 30 iterations 11.8 -> 3.45 -> 2.96 ms; four rounds' loads in flight need a second
+// wave of CTAs: 3.7 ms).
+// PARTS = 4: a quarter of a brick per warp, one round of loads instead of two, while all of the quarters are resident
+// (RB_SMALL_BRICKS): a frame of a 96x96x72 tank 1.19 -> 1.06 ms (half a brick 1.11); the large one 2.96 -> 3.76 ms.
+constexpr uint32_t RB_SMALL_BRICKS = 1480;  // their quarters are 148 SMs x RB_SMALL_CTAS x 8 warps
+constexpr int RB_SMALL_CTAS = 5;
+// Entry 2 t + 64 k of lane t in round k, its row y and plane z, and whether its red cells lie at odd x.
+struct RbGeo {
+    uint32_t i, h, y, z, odd;
+};
+__device__ __forceinline__ RbGeo rb_geo(uint32_t lane, uint32_t k) {
+    RbGeo g;
+    g.i = 2u * lane + 64u * k;
+    g.h = lane & 1u;
+    g.y = (lane >> 1) & 7u;
+    g.z = 2u * k + (lane >> 4);
+    g.odd = (g.y + g.z) & 1u;
+    return g;
+}
+__device__ __forceinline__ float2 rb_ld(const float* p) { return *reinterpret_cast<const float2*>(p); }
+__device__ __forceinline__ void rb_st(float* p, float a, float b) { *reinterpret_cast<float2*>(p) = make_float2(a, b); }
+// A half row's quad by colour: cells odd, odd + 2 are red.
+__device__ __forceinline__ void rb_put(float* dst, const RbGeo& g, const float4& v) {
+    rb_st(dst + g.i, g.odd ? v.y : v.x, g.odd ? v.w : v.z);
+    rb_st(dst + BRICK_CELLS / 2 + g.i, g.odd ? v.x : v.y, g.odd ? v.z : v.w);
+}
+// FIRST: the diagonals and words too (a frame's second solve has the same ones).
+template <bool FIRST>
+__global__ void __launch_bounds__(GRID_THREADS) k_rbgs_split(Dev d, MGState m, const float* __restrict__ pres, const float* __restrict__ rhs) {
+    pdl_entry();
+    const uint32_t active = d.active_bricks[0];
+    const uint32_t lane = threadIdx.x & 31u, wpb = blockDim.x >> 5;
+    uint8_t* words = reinterpret_cast<uint8_t*>(m.q);
+    for (uint32_t e = blockIdx.x * wpb + (threadIdx.x >> 5); e < active; e += gridDim.x * wpb) {
+        const uint32_t base = m.nbr_slots[8u * e + 6u] * BRICK_CELLS;
+#pragma unroll
+        for (uint32_t k = 0; k < 4u; ++k) {
+            const RbGeo g = rb_geo(lane, k);
+            const uint32_t c = base + 2u * g.i;  // the half row's first cell
+            rb_put(m.z + base, g, ld4(pres + c));
+            rb_put(m.r + base, g, ld4(rhs + c));
+            if (FIRST) {
+                const float4 dg = ld4(d.cell_diag + c);
+                uint32_t w4 = *reinterpret_cast<const uint32_t*>(m.word + c);
+                rb_put(m.dvec + base, g, dg);
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (!(comp(dg, j) > 0.0f)) w4 &= ~(W_FLUID << (8 * j));
+                const uint32_t even = (w4 & 0xFFu) | ((w4 >> 8) & 0xFF00u), odd = ((w4 >> 8) & 0xFFu) | ((w4 >> 16) & 0xFF00u);
+                *reinterpret_cast<uint16_t*>(words + base + g.i) = uint16_t(g.odd ? odd : even);
+                *reinterpret_cast<uint16_t*>(words + base + BRICK_CELLS / 2 + g.i) = uint16_t(g.odd ? even : odd);
+            }
+        }
+    }
+}
+__global__ void __launch_bounds__(GRID_THREADS) k_rbgs_merge(Dev d, MGState m, float* pres) {
+    pdl_entry();
+    const uint32_t active = d.active_bricks[0];
+    const uint32_t lane = threadIdx.x & 31u, wpb = blockDim.x >> 5;
+    for (uint32_t e = blockIdx.x * wpb + (threadIdx.x >> 5); e < active; e += gridDim.x * wpb) {
+        const uint32_t base = m.nbr_slots[8u * e + 6u] * BRICK_CELLS;
+#pragma unroll
+        for (uint32_t k = 0; k < 4u; ++k) {
+            const RbGeo g = rb_geo(lane, k);
+            const float2 r = rb_ld(m.z + base + g.i), b = rb_ld(m.z + base + BRICK_CELLS / 2 + g.i);
+            const float out[4] = {g.odd ? b.x : r.x, g.odd ? r.x : b.x, g.odd ? b.y : r.y, g.odd ? r.y : b.y};
+            st4(pres + base + 2u * g.i, out);
+        }
+    }
 }
 template <uint32_t PARTS>
-__global__ void __launch_bounds__(GRID_THREADS) k_rbgs(Dev d, MGState m, float* pres, const float* __restrict__ rhs, uint32_t parity, float omega) {
+__global__ void __launch_bounds__(GRID_THREADS) k_rbgs(Dev d, MGState m, uint32_t parity, float omega) {
     pdl_entry();
-    constexpr uint32_t B = 4u;
+    constexpr uint32_t B = PARTS == 4u ? 1u : 2u;  // rounds whose loads are in flight together
     const uint32_t active = PARTS * d.active_bricks[0];
     const uint32_t lane = threadIdx.x & 31u, wpb = blockDim.x >> 5;
+    const uint32_t own = parity * (BRICK_CELLS / 2), other = BRICK_CELLS / 2 - own;
     for (uint32_t t = blockIdx.x * wpb + (threadIdx.x >> 5); t < active; t += gridDim.x * wpb) {
-        const uint32_t e = t / PARTS, first = (8u / PARTS) * (t % PARTS);
+        const uint32_t e = t / PARTS, first = (4u / PARTS) * (t % PARTS);
         const uint4 s0 = *reinterpret_cast<const uint4*>(m.nbr_slots + 8u * e);
         const uint4 s1 = *reinterpret_cast<const uint4*>(m.nbr_slots + 8u * e + 4u);
-        const uint32_t ns[6] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y};
         const uint32_t base = s1.z * BRICK_CELLS;
+        const float* z = m.z + other;  // the other colour's entries of a brick start at its first cell
 #pragma unroll
-        for (uint32_t kk = 0; kk < 8u / PARTS; kk += B) {
-            const uint32_t k0 = first + kk;
+        for (uint32_t kk = 0; kk < 4u / PARTS; kk += B) {
             uint32_t w[B];
-            float b[B], dg[B], old[B], n[B][6];
+            float2 b[B], dg[B], old[B], c[B], n[B][4];
+            float x[B];
 #pragma unroll
             for (uint32_t j = 0; j < B; ++j) {
-                const uint32_t l = colour_local(lane, k0 + j, parity), i = base + l;
-                w[j] = m.word[i];
-                b[j] = rhs[i];
-                dg[j] = d.cell_diag[i];
-                old[j] = pres[i];
-#pragma unroll
-                for (int q = 0; q < 6; ++q) n[j][q] = pres[l0_nbr(i, l, q, ns)];
+                const RbGeo g = rb_geo(lane, first + kk + j);
+                const uint32_t i = base + g.i, off = g.odd ^ parity;
+                w[j] = *reinterpret_cast<const uint16_t*>(reinterpret_cast<const uint8_t*>(m.q) + own + i);
+                b[j] = rb_ld(m.r + own + i);
+                dg[j] = rb_ld(m.dvec + own + i);
+                old[j] = rb_ld(m.z + own + i);
+                c[j] = rb_ld(z + i);
+                // cells at even x (off 0) lack their left x neighbour in c, those at odd x the right one
+                x[j] = z[off == 0u ? (g.h ? i - 1u : s0.x * BRICK_CELLS + g.i + 3u) : (g.h ? s0.y * BRICK_CELLS + g.i - 2u : i + 2u)];
+                n[j][0] = rb_ld(z + (g.y > 0u ? i - 4u : s0.z * BRICK_CELLS + g.i + 28u));
+                n[j][1] = rb_ld(z + (g.y < 7u ? i + 4u : s0.w * BRICK_CELLS + g.i - 28u));
+                n[j][2] = rb_ld(z + (g.z > 0u ? i - 32u : s1.x * BRICK_CELLS + g.i + 224u));
+                n[j][3] = rb_ld(z + (g.z < 7u ? i + 32u : s1.y * BRICK_CELLS + g.i - 224u));
             }
 #pragma unroll
             for (uint32_t j = 0; j < B; ++j) {
-                if (!(w[j] & W_FLUID) || !(dg[j] > 0.0f)) continue;
-                float sum = 0.0f;
+                const RbGeo g = rb_geo(lane, first + kk + j);
+                const bool off = (g.odd ^ parity) != 0u;
+                float out[2] = {old[j].x, old[j].y};
 #pragma unroll
-                for (int q = 0; q < 6; ++q)
-                    if ((w[j] >> q) & 1u) sum = sum + n[j][q];
-                const float gs = (sum - b[j]) / dg[j];
-                pres[base + colour_local(lane, k0 + j, parity)] = old[j] + omega * (gs - old[j]);
+                for (int q = 0; q < 2; ++q) {
+                    const uint32_t wq = (w[j] >> (8 * q)) & 0xFFu;
+                    if (!(wq & W_FLUID)) continue;
+                    float sum = 0.0f;
+                    if (wq & 1u) sum = sum + (q ? (off ? c[j].y : c[j].x) : (off ? c[j].x : x[j]));
+                    if (wq & 2u) sum = sum + (q ? (off ? x[j] : c[j].y) : (off ? c[j].y : c[j].x));
+#pragma unroll
+                    for (int a = 0; a < 4; ++a)
+                        if (wq & (4u << a)) sum = sum + (q ? n[j][a].y : n[j][a].x);
+                    const float gs = (sum - (q ? b[j].y : b[j].x)) / (q ? dg[j].y : dg[j].x);
+                    out[q] = out[q] + omega * (gs - out[q]);
+                }
+                rb_st(m.z + own + base + g.i, out[0], out[1]);
             }
         }
     }
@@ -2702,14 +2784,16 @@ int launch_vcycle(const Dev& d, const MGState& m, int coarse_iterations, const S
     }
     return n;
 }
-int launch_rbgs_words(const Dev& d, const MGState& m, const Shape& sh, cudaStream_t s) {
-    launch_k(k_pcg_words, sh.mg_ctas, GRID_THREADS, 0, s, d, m);
-    return 1;
-}
-int launch_rbgs(const Dev& d, const MGState& m, float* pres, const float* rhs, uint32_t parity, float omega, uint32_t bricks, const Shape& sh,
+int launch_rbgs(const Dev& d, const MGState& m, float* pres, const float* rhs, int sweeps, float omega, bool first, uint32_t bricks, const Shape& sh,
                 cudaStream_t s) {
-    launch_k(bricks <= RB_HALF_BRICKS ? k_rbgs<2> : k_rbgs<1>, sh.mg_ctas, GRID_THREADS, 0, s, d, m, pres, rhs, parity, omega);
-    return 1;
+    if (first) launch_k(k_pcg_words, sh.mg_ctas, GRID_THREADS, 0, s, d, m);
+    launch_k(first ? k_rbgs_split<true> : k_rbgs_split<false>, sh.mg_ctas, GRID_THREADS, 0, s, d, m, pres, rhs);
+    const bool small = bricks <= RB_SMALL_BRICKS;
+    for (int it = 0; it < sweeps; ++it)
+        for (uint32_t colour = 0; colour < 2u; ++colour)
+            launch_k(small ? k_rbgs<4> : k_rbgs<1>, small ? sh.num_sms * RB_SMALL_CTAS : sh.mg_ctas, GRID_THREADS, 0, s, d, m, colour, omega);
+    launch_k(k_rbgs_merge, sh.mg_ctas, GRID_THREADS, 0, s, d, m, pres);
+    return (first ? 3 : 2) + 2 * std::max(sweeps, 0);
 }
 int launch_pcg_apply_a(const Dev& d, const MGState& m, const Shape& sh, cudaStream_t s) {
     if (mg_staged()) ST_LAUNCH(k_apply_a_st, 2, 1, d, m, sh, s);

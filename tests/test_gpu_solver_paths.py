@@ -34,6 +34,13 @@ def test_rbgs_matches_oracle(slosh, oracle_mod, grid, iterations):
     assert rg.last_solve_true_rel_residual == pytest.approx(ro.last_solve_true_rel_residual, rel=1e-6)
 
 
+# more bricks in the layout than the quarter-brick split takes: the first frame sweeps whole bricks
+def test_rbgs_whole_bricks_match_oracle(slosh, oracle_mod):
+    sc = _scene(slosh, (130, 96, 70), A.SOLVER_RBGS, pressure_iterations=3, density_projection_iterations=2, max_substeps=1)
+    g, o = pair(slosh, oracle_mod, sc)
+    run_frames(g, o, sc, frames=2, tol=None)
+
+
 # The cluster form of the solve (few active bricks) and the launched form against the oracle: one and two tail levels,
 # levels between level 0 and the tail, fixed counts and a tolerance, every preconditioner option, each storage precision.
 @pytest.mark.parametrize("grid", [(16, 16, 16), (21, 17, 30), (64, 40, 33), (96, 72, 50)])
