@@ -172,7 +172,11 @@ struct Ctx {
     SortBuffers sortb{};
     P2GGather gather{};  // the per-cell particle index of the gather P2G (allocated only when it is on)
     MGState mg{};
-    int cluster_most = 0;          // most CTAs of the solve's cluster form for this layout (0: not available)
+    // Most CTAs of the solve's cluster form for this layout (0: not available, -1: not asked yet). The question loads two
+    // kernels and takes 3 ms of about 30 of a context's creation, so a layout of more bricks than this asks when its tank
+    // first has few enough active ones.
+    static constexpr uint32_t CLUSTER_LAYOUT = 2048;
+    int cluster_most = 0;
     uint32_t bricks_estimate = 0;  // active bricks of the last frame; the layout's most before the first
 
     // pinned host staging
@@ -463,8 +467,8 @@ struct Ctx {
         total_emitted = 0;
         prev_dt = 0.0f;
         last_max_speed = 0.0f;
-        cluster_most = mg_solve_clusters(mg);
         bricks_estimate = num_pool_bricks - 1u;
+        cluster_most = bricks_estimate <= CLUSTER_LAYOUT ? mg_solve_clusters(mg) : -1;
         shape.num_sms = num_sms;
         shape.brick_ctas = brick_ctas_for(ctas_per_sm);
         shape.mg_ctas = brick_ctas_for(mg_ctas_per_sm);
@@ -721,6 +725,7 @@ struct Ctx {
         const Dev d = dev();
         // few active bricks: the whole solve in one cluster (the form does not change the result, so the last frame's
         // count, which the host has, is enough to choose by)
+        if (cluster_most < 0 && mg_solve_cluster(16, bricks_estimate) > 0) cluster_most = mg_solve_clusters(mg);
         const int cluster = mg_solve_cluster(cluster_most, bricks_estimate);
         SolveGraph* G = nullptr;
         if (use_graphs && cluster == 0) {

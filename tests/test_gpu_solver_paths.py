@@ -10,8 +10,8 @@ from parity import pair, run_frames
 pytestmark = pytest.mark.gpu
 
 
-def _scene(slosh, grid, solver, **settings):
-    mn, dims = scenes.box_cells(grid, (0.0, 0.0, 0.0), (0.45, 0.6, 1.0))
+def _scene(slosh, grid, solver, fill=(0.45, 0.6, 1.0), **settings):
+    mn, dims = scenes.box_cells(grid, (0.0, 0.0, 0.0), fill)
     count = dims[0] * dims[1] * dims[2] * 8
     s = scenes.base_settings(slosh.settings_default, grid, count)
     s.cell_size = 1.0 / max(grid)
@@ -55,3 +55,10 @@ def test_mgpcg_forms_match_oracle(slosh, oracle_mod, grid, settings):
     sc = _scene(slosh, grid, A.SOLVER_MGPCG, **settings)
     g, o = pair(slosh, oracle_mod, sc)
     run_frames(g, o, sc, frames=2, tol=None)
+
+
+# a layout of many bricks with few active ones: launched first, one cluster from the second frame on
+def test_mgpcg_few_bricks_of_a_large_layout_match_oracle(slosh, oracle_mod):
+    sc = _scene(slosh, (136, 136, 72), A.SOLVER_MGPCG, fill=(0.2, 0.25, 0.4), tolerance=1e-6, max_substeps=1)
+    g, o = pair(slosh, oracle_mod, sc)
+    run_frames(g, o, sc, frames=3, tol=None)
