@@ -16,7 +16,10 @@
 //   * levels 1-3 are visited through the active bricks' footprints (a brick covers (8 >> l)^3 cells
 //     of level l), not by scanning the dense level; every fluid coarse cell lies in such a footprint;
 //   * the small coarse levels (<= 4096 cells) run as one single-CTA kernel (descent, coarse solve,
-//     ascent with block barriers between passes).
+//     ascent with block barriers between passes); the levels between level 0 or 1 and them take one pass each
+//     way (k_coarse_down, k_coarse_up);
+//   * a tank of few active bricks runs the whole solve in one thread-block cluster (mg_cluster.cuh).
+// The red-black SOR solver (k_rbgs) sweeps over the same stencil words.
 #include <algorithm>
 #include <cstdlib>
 
