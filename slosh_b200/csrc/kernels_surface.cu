@@ -16,6 +16,7 @@
 #include <cuda_fp16.h>
 
 #include "kernels.h"
+#include "splat_box.h"
 
 namespace slosh {
 
@@ -87,27 +88,14 @@ __device__ __forceinline__ SplatShape splat_shape(const SurfaceDev& s) {
     h.small = fabsf(s.radius_voxels) < 8192.0f;
     return h;
 }
-// The voxels a particle visits. The reference's box reaches one voxel beyond the kernel on each side; where the
-// kernel is not cut by the footprint those (more than 1e-3 kernel radii outside) fail the distance test, and are left
-// out: 2-3 voxels an axis instead of 4-5 at the default kernel.
+// The voxels a particle visits (splat_span): 2-3 voxels an axis instead of the reference's 4-5 at the default kernel.
 __device__ __forceinline__ SplatKernel splat_kernel(const SurfaceDev& s, const SplatShape& h, float4 a) {
     SplatKernel k;
     k.c = make_float3(a.x * s.inv_voxel, a.y * s.inv_voxel, a.z * s.inv_voxel);
-    const float3 c = k.c;
-    const float rr = h.reach;
-    k.lo = make_int3(max(int(floorf(c.x - rr - 0.5f)), 0), max(int(floorf(c.y - rr - 0.5f)), 0), max(int(floorf(c.z - rr - 0.5f)), 0));
-    k.hi = make_int3(min(int(ceilf(c.x + rr - 0.5f)), s.dim.x - 1), min(int(ceilf(c.y + rr - 0.5f)), s.dim.y - 1),
-                     min(int(ceilf(c.z + rr - 0.5f)), s.dim.z - 1));
-    if (h.whole) {
-        const float far = rr * 1.001f;  // the test squares this same difference times 1 / rr
-        auto cut = [&](int& lo, int& hi, float x) {
-            if ((float(lo) + 0.5f) - x < -far) ++lo;
-            if ((float(hi) + 0.5f) - x > far) --hi;
-        };
-        cut(k.lo.x, k.hi.x, c.x);
-        cut(k.lo.y, k.hi.y, c.y);
-        cut(k.lo.z, k.hi.z, c.z);
-    }
+    const SplatSpan x = splat_span(k.c.x, h.reach, s.dim.x, h.whole), y = splat_span(k.c.y, h.reach, s.dim.y, h.whole),
+                    z = splat_span(k.c.z, h.reach, s.dim.z, h.whole);
+    k.lo = make_int3(x.lo, y.lo, z.lo);
+    k.hi = make_int3(x.hi, y.hi, z.hi);
     return k;
 }
 // x rounded to the nearest integer (ties to even) for |x| < 2^22, and cut to an integer for 0 <= x < 2^22: the sum

@@ -45,3 +45,30 @@ def test_splat_paths_match_oracle(slosh, oracle_mod, grid, res, smooth, order, c
     q = S.surface_params_default()
     q.field_resolution, q.surface_smoothing = res, smooth
     _compare(g, o, q)
+
+
+# live records at infinite, NaN and far positions have no voxel: the field is the one without them, in kernels of three
+# voxels, wider ones and ones that the footprint cuts
+@pytest.mark.parametrize("res,smooth", [(1.0, 2.0), (1.5, 2.0), (1.5, 3.0), (3.0, 6.0)])
+def test_splat_leaves_out_far_records(slosh, oracle_mod, res, smooth):
+    grid = (24, 20, 28)
+    s = slosh.settings_default()
+    s.grid_dim[:] = list(grid)
+    s.cell_size = 1.0 / max(grid)
+    s.particle_capacity = 8192
+    rec = _records(grid, 1500, "sorted", 5)
+    far = [np.inf, -np.inf, np.nan, 1e30, -1e30] + [v * s.cell_size / res for v in (2.0 ** 31, -(2.0 ** 31), 2.0 ** 31 + 512.0, 1e9)]
+    bad = np.zeros(3 * len(far) + 1, S.PARTICLE_DTYPE)
+    bad["pos"] = 0.4
+    for k, v in enumerate(far):
+        for a in range(3):
+            bad["pos"][3 * k + a, a] = v
+    bad["pos"][-1] = np.inf
+    bad["age"] = 1.0
+    both = np.concatenate([rec[:700], bad, rec[700:]])
+    q = S.surface_params_default()
+    q.field_resolution, q.surface_smoothing = res, smooth
+    g, o = slosh.Simulation(s), oracle_mod.Oracle(s)
+    g.upload_particles(both)
+    o.upload_particles(rec)
+    _compare(g, o, q)
