@@ -9,6 +9,7 @@
 // and independent of the order in which particles add them.
 #include <cstdlib>
 
+#include "g2p_box.h"
 #include "kernels.h"
 
 namespace slosh {
@@ -720,13 +721,14 @@ struct TileField {
         bool in = true;
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
+            int first[2];
 #pragma unroll
             for (int v = 0; v < 2; ++v) {
                 const float gv = g[a] - (v ? 0.5f : 0.0f), fl = floorf(gv);
-                q.b[a][v] = int(fl) - o[a];
+                first[v] = int(fl);
                 q.f[a][v] = gv - fl;
             }
-            in = in && q.b[a][1] >= 0 && q.b[a][0] < n[a] - 1;  // the stencil beside starts no later and ends no later
+            in = tile_axis(first[0], first[1], o[a], n[a], q.b[a]) && in;
         }
         return in;
     }
