@@ -10,14 +10,11 @@
 
 namespace slosh {
 
-// b0, b1: the first nodes of the stencils for a face on the axis and beside it (b1 is b0 or b0 - 1; saturated integers for
-// far positions); the tile has the n nodes from o on, o + n below 2^30. True when both stencils' nodes lie in the tile; local
-// then holds the first nodes' places in it. The differences are taken modulo 2^32, where b0's of any node outside the tile is
-// at least n - 1.
-SLOSH_HD bool tile_axis(int b0, int b1, int o, int n, int (&local)[2]) {
-    local[0] = int(unsigned(b0) - unsigned(o));
-    local[1] = int(unsigned(b1) - unsigned(o));
-    return local[1] >= 0 && unsigned(local[0]) < unsigned(n - 1);  // the stencil beside starts no later and ends no later
-}
+// The place of node b in a tile that starts at node o, modulo 2^32: of a far position b has saturated, and b - o may wrap.
+SLOSH_HD int tile_place(int b, int o) { return int(unsigned(b) - unsigned(o)); }
+// Whether both stencils' nodes lie in the tile of n nodes; l0, l1: the places of the first nodes of the stencils for a face on
+// the axis and beside it, which are nodes b and b, or b and b - 1 within +-2^30 (farther out half a cell changes no float). With
+// o + n below 2^30 a place that wraps comes out above every n, which fails the second test.
+SLOSH_HD bool tile_holds(int l0, int l1, int n) { return l1 >= 0 && l0 < n - 1; }
 
 }  // namespace slosh

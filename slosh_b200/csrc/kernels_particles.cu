@@ -721,14 +721,13 @@ struct TileField {
         bool in = true;
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-            int first[2];
 #pragma unroll
             for (int v = 0; v < 2; ++v) {
                 const float gv = g[a] - (v ? 0.5f : 0.0f), fl = floorf(gv);
-                first[v] = int(fl);
+                q.b[a][v] = tile_place(int(fl), o[a]);
                 q.f[a][v] = gv - fl;
             }
-            in = tile_axis(first[0], first[1], o[a], n[a], q.b[a]) && in;
+            in = in && tile_holds(q.b[a][0], q.b[a][1], n[a]);
         }
         return in;
     }
