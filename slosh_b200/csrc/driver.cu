@@ -844,13 +844,13 @@ struct Ctx {
             count(launch_clear_new_slots(d, shape, stream));
         }
         float* V[3] = {vel[vmap[0]], vel[vmap[1]], vel[vmap[2]]};
+        const bool unsorted = placed_since_sort * 8u > num_particles;  // more than an eighth of the particles in placement order
         {
             PhaseScope ps(this, 2);
             if (p2g_gather_enabled()) {
                 count(launch_p2g_gather(d, P, gather, particles[pbuf], num_particles, stream));
             } else {
-                // more than an eighth of the particles in placement order: the wider P2G tile
-                count(launch_p2g(d, P, particles[pbuf], num_particles, placed_since_sort * 8u > num_particles, stream));
+                count(launch_p2g(d, P, particles[pbuf], num_particles, unsorted, stream));
             }
         }
         int c = 0;
@@ -912,7 +912,7 @@ struct Ctx {
         }
         {
             PhaseScope ps(this, 8);
-            count(launch_g2p(d, P, particles[pbuf], num_particles, V[c], V[(c + 2) % 3], density, stream));
+            count(launch_g2p(d, P, particles[pbuf], num_particles, V[c], V[(c + 2) % 3], density, unsorted, stream));
         }
         // The field of logical buffer c becomes logical buffer 0 for the next substep.
         const int nm[3] = {vmap[c], vmap[(c + 1) % 3], vmap[(c + 2) % 3]};

@@ -58,3 +58,38 @@ def test_transfers_match_oracle(slosh, oracle_mod, count, order, speed, transfer
             assert not bad, bad
         g.end_frame()
         o.end_frame()
+
+
+# the same records once sorted (the shared-memory tile, which unsorted ones do not take), and a frame after which they are
+# in placement order again (the pool)
+@pytest.mark.parametrize("density", [0, 1])
+@pytest.mark.parametrize("order,speed", [("sorted", 0.5), ("outside", 0.5), ("sorted", 12.0)])
+@pytest.mark.parametrize("count", [383, 385, 9000])
+def test_apic_after_a_sort_matches_oracle(slosh, oracle_mod, count, order, speed, density):
+    grid = (30, 24, 21)
+    s = slosh.settings_default()
+    s.grid_dim[:] = list(grid)
+    s.cell_size = 1.0 / max(grid)
+    s.particle_capacity = 16384
+    s.min_substeps = s.max_substeps = 2
+    s.max_speed = 40.0
+    s.two_sided_density_projection = density
+    s.sort_interval = 2
+    g, o = slosh.Simulation(s), oracle_mod.Oracle(s)
+    rec = _records(grid, count, order, speed, count)
+    for sim in (g, o):
+        sim.upload_particles(rec)
+    fi = A.frame_input(s, delta_time=1.0 / 60.0)
+    for f in range(3):
+        if f == 2:
+            rec = g.particles()[::-1].copy()
+            for sim in (g, o):
+                sim.upload_particles(rec)
+        assert g.begin_frame(fi) == o.begin_frame(fi)
+        for k in range(2):
+            g.substep(k)
+            o.substep(k)
+            bad = compare_state(g, o).failures()
+            assert not bad, bad
+        g.end_frame()
+        o.end_frame()
