@@ -1018,7 +1018,7 @@ void Ctx::build_surface(const slosh_surface_params_t& q) {
         d.indices = salloc<uint32_t>(q.max_indices);
         d.counters = salloc<uint32_t>(2);
     }
-    count(launch_surface(d, particles[pbuf], num_particles, q.build_mesh != 0u, stream));
+    count(launch_surface(d, particles[pbuf], num_particles, q.build_mesh != 0u, num_sms, stream));
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(h_surf, d.counters, 8, cudaMemcpyDeviceToHost, stream));
     d2h_bytes += 8;

@@ -196,6 +196,6 @@ struct SurfaceDev {
     uint32_t* counters;     // [0] vertices requested, [1] indices requested
 };
 // Splat, resolve and (with mesh) surface nets of the first n particle records.
-int launch_surface(const SurfaceDev& s, const slosh_particle_t* particles, uint32_t n, bool mesh, cudaStream_t st);
+int launch_surface(const SurfaceDev& s, const slosh_particle_t* particles, uint32_t n, bool mesh, int num_sms, cudaStream_t st);
 
 }  // namespace slosh

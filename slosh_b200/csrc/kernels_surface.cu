@@ -49,7 +49,7 @@ __device__ __forceinline__ float dot3f(float3 a, float3 b) { return a.x * b.x + 
 // into one square per axis: q2 = (x^2 + y^2) + z^2, the reference's three dot products with their zero terms left
 // out (adding a zero changes no bit of a square); a row of voxels with y^2 + z^2 >= 1 has no voxel inside, because
 // rounding is monotonic.
-// One CTA takes SPLAT_CHUNK consecutive (spatially sorted) particles, adds their moments into a shared-memory tile
+// One CTA takes PER x 256 consecutive (spatially sorted) particles, adds their moments into a shared-memory tile
 // over the bounding box of their kernels and adds each non-zero tile word to global memory once. A box larger than
 // the tile is visited in slabs of whole z planes (every particle adds the rows of its kernel that lie in the slab);
 // more than SPLAT_MAX_SLABS slabs (particles in no spatial order) add straight to global memory.
@@ -58,14 +58,13 @@ __device__ __forceinline__ float dot3f(float3 a, float3 b) { return a.x * b.x + 
 // 8.2 M particles in 160^3 voxels, the default kernel: 1,857 us with global atomics, 529 with the tile, 467 with the
 // voxels taken from a mask, about 375 with the 27 tests of a small kernel from nine squares. A field with its mesh:
 // 2,349 -> 632 us there, 366 -> 182 us for 64 x 64 x 48 voxels and 0.7 M particles. 4 CTAs per SM (64 registers);
-// 1 particle per thread or a tile of 1,536 voxels took 655 us, 4 per thread in CTAs of 128 took 706, chunks of 2,048
+// 1 particle per thread (at this size) or a tile of 1,536 voxels took 655 us, 4 per thread in CTAs of 128 took 706, chunks of 2,048
 // and 4,096 particles (before the small kernel's form) 904 and 953 against 726: too few warps in flight.
 constexpr int SPLAT_THREADS = 256;
-constexpr int SPLAT_PER_THREAD = 2;
-constexpr int SPLAT_CHUNK = SPLAT_THREADS * SPLAT_PER_THREAD;  // about one 4^3 sort key of 8 particles a cell
-constexpr int SPLAT_TILE = 2048;                               // voxels: 40 KB, 5 CTAs per SM
+constexpr int SPLAT_CTAS = 4;  // per SM
+constexpr int SPLAT_TILE = 2048;                               // voxels: 40 KB
 constexpr int SPLAT_SMEM = SPLAT_TILE * int(FIELD_MOMENTS) * 4;
-constexpr int SPLAT_MAX_SLABS = 8;
+template <int PER> constexpr int SPLAT_MAX_SLABS = PER == 1 ? 4 : 8;
 
 struct SplatKernel {
     float3 c;  // the particle in voxels
@@ -219,21 +218,26 @@ __device__ __forceinline__ void splat_voxels(const SurfaceDev& s, const SplatSha
         }
     }
 }
-__global__ void __launch_bounds__(SPLAT_THREADS, 4) k_density_splat(SurfaceDev s, const slosh_particle_t* __restrict__ particles, uint32_t n) {
+// PER: particles per thread. 2 (a CTA's 512 are about one 4^3 sort key of 8 a cell) for many; 1 while all of those CTAs run at
+// once, where a second particle, or a fifth slab, is only a longer chain. A field alone, us with global atomics, with 2 per
+// thread, with 1 (and 8 slabs): 2,000 records all over 64^3 voxels, smoothing 6, 224, 348, 199; 20,000 in a sorted sheet, 96^3
+// voxels, smoothing 3, 143, 276, 104 (165); 100,000 sorted, 64^3 voxels, smoothing 6, 762, 347, 243 (240).
+template <int PER>
+__global__ void __launch_bounds__(SPLAT_THREADS, SPLAT_CTAS) k_density_splat(SurfaceDev s, const slosh_particle_t* __restrict__ particles, uint32_t n) {
     extern __shared__ int32_t splat_tile[];  // [5][SPLAT_TILE]
     __shared__ int s_box[6];
     const int big = 0x7FFFFFFF;
     if (threadIdx.x < 3) { s_box[threadIdx.x] = big; s_box[3 + threadIdx.x] = -big; }
     __syncthreads();
     const SplatShape shape = splat_shape(s);
-    SplatKernel kern[SPLAT_PER_THREAD];
-    bool live[SPLAT_PER_THREAD];
+    constexpr int CHUNK = SPLAT_THREADS * PER;
+    SplatKernel kern[PER];
+    bool live[PER];
     int3 mn = make_int3(big, big, big), mx = make_int3(-big, -big, -big);
 #pragma unroll
-    for (int j = 0; j < SPLAT_PER_THREAD; ++j) {
-        // lanes 16 records apart: neighbouring records share a cell, and lanes adding to one voxel take turns
-        const uint32_t i = blockIdx.x * uint32_t(SPLAT_CHUNK) + (threadIdx.x & 31u) * uint32_t(SPLAT_CHUNK / 32) +
-                           (threadIdx.x >> 5) * uint32_t(SPLAT_PER_THREAD) + uint32_t(j);
+    for (int j = 0; j < PER; ++j) {
+        // lanes 8 PER records apart: neighbouring records share a cell, and lanes adding to one voxel take turns
+        const uint32_t i = blockIdx.x * uint32_t(CHUNK) + (threadIdx.x & 31u) * uint32_t(CHUNK / 32) + (threadIdx.x >> 5) * uint32_t(PER) + uint32_t(j);
         const float4 a = i < n ? __ldg(reinterpret_cast<const float4*>(particles + i)) : make_float4(0.0f, 0.0f, 0.0f, -1.0f);
         kern[j] = splat_kernel(s, shape, a);
         // a removed particle's ellipsoid is all zeros: skipped; a kernel outside the field touches no voxel
@@ -255,9 +259,9 @@ __global__ void __launch_bounds__(SPLAT_THREADS, 4) k_density_splat(SurfaceDev s
     const int3 e = make_int3(s_box[3] - o.x + 1, s_box[4] - o.y + 1, s_box[5] - o.z + 1);
     const long long plane = (long long)e.x * e.y;
     const int rows = plane <= SPLAT_TILE ? int(SPLAT_TILE / plane) : 0;  // z planes of a slab
-    if (rows == 0 || e.z > rows * SPLAT_MAX_SLABS) {
+    if (rows == 0 || e.z > rows * SPLAT_MAX_SLABS<PER>) {
 #pragma unroll
-        for (int j = 0; j < SPLAT_PER_THREAD; ++j)
+        for (int j = 0; j < PER; ++j)
             if (live[j])
                 splat_voxels(s, shape, kern[j], kern[j].lo.z, kern[j].hi.z, [&](int x, int y, int z, const int32_t* m) {
                     int32_t* acc = s.accum + voxel_index(s, make_int3(x, y, z)) * FIELD_MOMENTS;
@@ -276,7 +280,7 @@ __global__ void __launch_bounds__(SPLAT_THREADS, 4) k_density_splat(SurfaceDev s
         }
         __syncthreads();
 #pragma unroll
-        for (int j = 0; j < SPLAT_PER_THREAD; ++j)
+        for (int j = 0; j < PER; ++j)
             if (live[j])
                 splat_voxels(s, shape, kern[j], o.z + z0, o.z + z0 + nz - 1, [&](int x, int y, int z, const int32_t* m) {
                     int32_t* acc = splat_tile + (x - o.x) + e.x * (y - o.y) + int(pl) * (z - o.z - z0);
@@ -493,7 +497,7 @@ int blocks_of(uint64_t n) { return int((n + SURF_THREADS - 1) / SURF_THREADS); }
 
 }  // namespace
 
-int launch_surface(const SurfaceDev& s, const slosh_particle_t* particles, uint32_t n, bool mesh, cudaStream_t st) {
+int launch_surface(const SurfaceDev& s, const slosh_particle_t* particles, uint32_t n, bool mesh, int num_sms, cudaStream_t st) {
     const uint64_t nv = uint64_t(s.dim.x) * uint64_t(s.dim.y) * uint64_t(s.dim.z);
     const uint64_t nb = uint64_t(s.bdim.x) * uint64_t(s.bdim.y) * uint64_t(s.bdim.z);
     int launches = 0;
@@ -501,9 +505,12 @@ int launch_surface(const SurfaceDev& s, const slosh_particle_t* particles, uint3
     cudaMemsetAsync(s.bricks, 0, nb * 4, st);
     cudaMemsetAsync(s.counters, 0, 8, st);
     if (n > 0) {
+        const bool few = n <= uint32_t(num_sms * SPLAT_CTAS * SPLAT_THREADS);
+        const uint32_t chunk = SPLAT_THREADS * (few ? 1u : 2u);
+        auto kernel = few ? k_density_splat<1> : k_density_splat<2>;
         // room for four CTAs' tiles per SM
-        cudaFuncSetAttribute(k_density_splat, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-        k_density_splat<<<int((uint64_t(n) + SPLAT_CHUNK - 1) / SPLAT_CHUNK), SPLAT_THREADS, SPLAT_SMEM, st>>>(s, particles, n);
+        cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        kernel<<<int((uint64_t(n) + chunk - 1u) / chunk), SPLAT_THREADS, SPLAT_SMEM, st>>>(s, particles, n);
         ++launches;
     }
     k_field_resolve<<<blocks_of(nv), SURF_THREADS, 0, st>>>(s);

@@ -72,3 +72,21 @@ def test_splat_leaves_out_far_records(slosh, oracle_mod, res, smooth):
     g.upload_particles(both)
     o.upload_particles(rec)
     _compare(g, o, q)
+
+
+# more particles than a wave of CTAs with one particle per thread: two per thread, up to eight slabs
+@pytest.mark.parametrize("order", ["sorted", "random"])
+@pytest.mark.parametrize("res,smooth", [(1.0, 2.0), (1.5, 3.0)])
+def test_splat_of_many_records_matches_oracle(slosh, oracle_mod, res, smooth, order):
+    grid = (50, 64, 39)
+    s = slosh.settings_default()
+    s.grid_dim[:] = list(grid)
+    s.cell_size = 1.0 / max(grid)
+    s.particle_capacity = 200000
+    rec = _records(grid, 190001, order, 7)
+    g, o = slosh.Simulation(s), oracle_mod.Oracle(s)
+    for sim in (g, o):
+        sim.upload_particles(rec)
+    q = S.surface_params_default()
+    q.field_resolution, q.surface_smoothing = res, smooth
+    _compare(g, o, q)
