@@ -62,3 +62,20 @@ def test_mgpcg_few_bricks_of_a_large_layout_match_oracle(slosh, oracle_mod):
     sc = _scene(slosh, (136, 136, 72), A.SOLVER_MGPCG, fill=(0.2, 0.25, 0.4), tolerance=1e-6, max_substeps=1)
     g, o = pair(slosh, oracle_mod, sc)
     run_frames(g, o, sc, frames=3, tol=None)
+
+
+def _launches(g, fi):
+    before = g.launch_count()
+    g.step_frame(fi)
+    return g.launch_count() - before
+
+
+# Launches of a frame of one substep with 6 + 2 solver iterations: two cluster kernels and about 30 others, or more than ten an
+# iteration. A level-4 tail (more than 4,096 cells at level 3) has no resident form and must not take the cluster.
+@pytest.mark.parametrize("grid,cluster", [((128, 128, 120), True), ((136, 136, 136), False)])
+def test_few_bricks_take_the_cluster_where_it_is_resident(slosh, oracle_mod, grid, cluster):
+    sc = _scene(slosh, grid, A.SOLVER_MGPCG, fill=(0.1, 0.12, 0.1), pcg_iterations=6, max_substeps=1, mg_smoothing_sweeps=2)
+    g, o = pair(slosh, oracle_mod, sc)
+    run_frames(g, o, sc, frames=2, tol=None)
+    n = _launches(g, A.frame_input(sc["settings"]))
+    assert n < 50 if cluster else n > 90, n
