@@ -177,7 +177,18 @@ struct Ctx {
     // first has few enough active ones.
     static constexpr uint32_t CLUSTER_LAYOUT = 2048;
     int cluster_most = 0;
-    uint32_t bricks_estimate = 0;  // active bricks of the last frame; the layout's most before the first
+    // What the host knows of the active bricks (expected_bricks): the last stepped frame's most, or the layout's before the first
+    // one and after records or state were written from outside; and the bricks that emissions since then can wake.
+    uint32_t bricks_last = 0;
+    struct Emitted {
+        int lo[3], hi[3];          // the emissions' common box of bricks, with the layer around it that the pool keeps
+        uint64_t count, bricks;    // particles; sum of the single emissions' bounds
+        uint64_t volume(const Emitted& o) const {  // bricks of the box that lie in o's
+            uint64_t v = count && o.count ? 1u : 0u;
+            for (int a = 0; a < 3; ++a) v *= uint64_t(std::max(std::min(hi[a], o.hi[a]) - std::max(lo[a], o.lo[a]) + 1, 0));
+            return v;
+        }
+    } emitted{}, emitted_before{};  // since the last stepped frame; before it and in it
 
     // pinned host staging
     slosh_collider_t* h_colliders = nullptr;
@@ -467,8 +478,8 @@ struct Ctx {
         total_emitted = 0;
         prev_dt = 0.0f;
         last_max_speed = 0.0f;
-        bricks_estimate = num_pool_bricks - 1u;
-        cluster_most = bricks_estimate <= CLUSTER_LAYOUT ? mg_solve_clusters(mg) : -1;
+        forget_bricks();
+        cluster_most = bricks_last <= CLUSTER_LAYOUT ? mg_solve_clusters(mg) : -1;
         shape.num_sms = num_sms;
         shape.brick_ctas = brick_ctas_for(ctas_per_sm);
         shape.mg_ctas = brick_ctas_for(mg_ctas_per_sm);
@@ -640,6 +651,55 @@ struct Ctx {
         total_emitted += cnt;
         num_particles += uint32_t(cnt);
         placed_since_sort += cnt;
+        note_emitted(em, cnt);
+    }
+
+    // The box of bricks that an emission's cnt particles can wake: the positions k_emit forms, a cell around them for
+    // rounding, and the layer of bricks around touched ones that the pool update keeps. A particle wakes at most 27.
+    void note_emitted(const slosh_emit_request_t& em, uint64_t cnt) {
+        Emitted e{};
+        e.count = cnt;
+        double turn = 1.0, reach = 0.0;  // a box's corners may turn anywhere; a quaternion that is not of unit length scales them too
+        const double qv = std::sqrt(double(em.rotation[0]) * em.rotation[0] + double(em.rotation[1]) * em.rotation[1] + double(em.rotation[2]) * em.rotation[2]);
+        const double qw = std::fabs(double(em.rotation[3]));
+        if (std::fabs(qv * qv + qw * qw - 1.0) > 1e-3) turn = 1.0 + 2.0 * qv * (qw + qv);
+        for (int a = 0; a < 3; ++a) reach += double(em.extent[a]) * em.extent[a];
+        reach = (em.shape == SLOSH_EMIT_SPHERE ? std::fabs(double(em.extent[0])) : std::sqrt(reach) * turn) / S.cell_size;
+        const int bricks[3] = {brick_dim.x, brick_dim.y, brick_dim.z};
+        for (int a = 0; a < 3; ++a) {
+            double lo = double(em.center[a]) / S.cell_size - reach, hi = double(em.center[a]) / S.cell_size + reach;
+            if (em.shape == SLOSH_EMIT_FILL_CELLS) {
+                const double j = 0.25 * std::fabs(double(em.fill_jitter));
+                lo = double(em.cell_min[a]) - j;
+                hi = double(em.cell_min[a]) + double(em.cell_dims[a]) + j;
+            }
+            // (not a number: the whole axis)
+            const double most = double(bricks[a] - 1);
+            e.lo[a] = lo == lo ? int(std::min(std::max(std::floor((lo - 1.0) / 8.0) - 1.0, 0.0), std::max(most - 1.0, 0.0))) : 0;
+            e.hi[a] = hi == hi ? int(std::max(std::min(std::floor((hi + 1.0) / 8.0) + 1.0, most), std::min(1.0, most))) : bricks[a] - 1;
+        }
+        e.bricks = std::min(e.volume(e), 27u * cnt);
+        if (emitted.count == 0) {
+            emitted = e;
+            return;
+        }
+        for (int a = 0; a < 3; ++a) {
+            emitted.lo[a] = std::min(emitted.lo[a], e.lo[a]);
+            emitted.hi[a] = std::max(emitted.hi[a], e.hi[a]);
+        }
+        emitted.count += e.count;
+        emitted.bricks += e.bricks;
+    }
+    void forget_bricks() {
+        bricks_last = num_pool_bricks - 1u;
+        emitted = emitted_before = Emitted{};
+    }
+    // About how many bricks the coming solves have (at most; tanks also grow by flowing). A steady emitter's box holds the bricks
+    // that its last emission woke, which the last frame has counted.
+    uint32_t expected_bricks() const {
+        uint64_t more = emitted.volume(emitted);
+        if (emitted.count <= 2u * emitted_before.count) more -= emitted.volume(emitted_before);
+        return uint32_t(std::min<uint64_t>(bricks_last + std::min(more, emitted.bricks), num_pool_bricks - 1u));
     }
 
     void sort_particles() {
@@ -723,10 +783,11 @@ struct Ctx {
         const bool tol_mode = fixed_iterations <= 0;
         const uint32_t limit = tol_mode ? uint32_t(std::max(max_iterations, 1)) : uint32_t(std::min(std::max(fixed_iterations, 1), 100));
         const Dev d = dev();
-        // few active bricks: the whole solve in one cluster (the form does not change the result, so the last frame's
-        // count, which the host has, is enough to choose by)
-        if (cluster_most < 0 && mg_solve_cluster(16, bricks_estimate) > 0) cluster_most = mg_solve_clusters(mg);
-        const int cluster = mg_solve_cluster(cluster_most, bricks_estimate);
+        // few active bricks: the whole solve in one cluster (the form does not change the result, so what the host knows is
+        // enough to choose by)
+        const uint32_t bricks = expected_bricks();
+        if (cluster_most < 0 && mg_solve_cluster(16, bricks) > 0) cluster_most = mg_solve_clusters(mg);
+        const int cluster = mg_solve_cluster(cluster_most, bricks);
         SolveGraph* G = nullptr;
         if (use_graphs && cluster == 0) {
             try {
@@ -882,7 +943,7 @@ struct Ctx {
                 else mgpcg(pressure, divergence, S.pcg_iterations, 0.0f, 0, coarse, 0);
             } else {
                 const float omega = clampf_h(S.sor_weight, 0.5f, 1.95f);
-                count(launch_rbgs(d, mg, pressure, divergence, S.pressure_iterations, omega, true, bricks_estimate, shape, stream));
+                count(launch_rbgs(d, mg, pressure, divergence, S.pressure_iterations, omega, true, expected_bricks(), shape, stream));
                 last_iterations = S.pressure_iterations;
                 last_converged = true;
             }
@@ -901,7 +962,7 @@ struct Ctx {
             if (S.pressure_solver == SLOSH_SOLVER_MGPCG) {
                 mgpcg(density_q, density_rhs, 2, 0.0f, 0, clampi_h(S.mg_coarse_iterations, 1, 200), 1);
             } else {
-                count(launch_rbgs(d, mg, density_q, density_rhs, std::max(S.density_projection_iterations, 1), 1.7f, false, bricks_estimate, shape, stream));
+                count(launch_rbgs(d, mg, density_q, density_rhs, std::max(S.density_projection_iterations, 1), 1.7f, false, expected_bricks(), shape, stream));
             }
         }
         {
@@ -952,7 +1013,9 @@ void Ctx::end_frame_enqueue() {
 void Ctx::end_frame_finish() {
     CK(cudaStreamSynchronize(stream));
     if (substeps > 0) {
-        bricks_estimate = h_stats[7];
+        bricks_last = h_stats[7];
+        emitted_before = emitted;
+        emitted = Emitted{};
         float ms;
         std::memcpy(&ms, &h_stats[0], 4);
         last_max_speed = std::isfinite(ms) ? ms : 0.0f;
@@ -1459,6 +1522,7 @@ SLOSH_API slosh_status slosh_upload_particles(void* ctx, const slosh_particle_t*
             CK(cudaMemcpyAsync(c->particles[c->pbuf], particles, sizeof(slosh_particle_t) * count, cudaMemcpyHostToDevice, c->stream));
         c->num_particles = count;
         c->placed_since_sort = count;
+        c->forget_bricks();
         uint32_t pcv[2] = {count, 0u};
         CK(cudaMemcpyAsync(c->particle_count, pcv, 8, cudaMemcpyHostToDevice, c->stream));
         c->h2d_bytes += sizeof(slosh_particle_t) * count + 8;
@@ -1589,6 +1653,7 @@ SLOSH_API slosh_status slosh_write_buffer(void* ctx, int32_t buffer_id, const vo
         Ctx* c = as_ctx(ctx);
         if (buffer_id < 0 || buffer_id >= SLOSH_BUF_COUNT_) throw StatusError{SLOSH_ERR_INVALID_ARG, "bad buffer id"};
         CK(cudaStreamSynchronize(c->stream));
+        if (buffer_id == SLOSH_BUF_PARTICLES || (buffer_id >= SLOSH_BUF_BRICK_TABLE && buffer_id <= SLOSH_BUF_BRICK_TOUCH)) c->forget_bricks();
         if (buffer_id == SLOSH_BUF_PARTICLES) {
             const size_t n = bytes / sizeof(slosh_particle_t);
             if (n > c->capacity) throw StatusError{SLOSH_ERR_CAPACITY, "more particles than particle_capacity"};

@@ -79,3 +79,51 @@ def test_few_bricks_take_the_cluster_where_it_is_resident(slosh, oracle_mod, gri
     run_frames(g, o, sc, frames=2, tol=None)
     n = _launches(g, A.frame_input(sc["settings"]))
     assert n < 50 if cluster else n > 90, n
+
+
+def _drop_and_block(slosh):
+    """A tank of 1,152 bricks with a drop in it that wakes 27 of them, and a block that wakes more than a cluster holds."""
+    grid = (96, 96, 64)
+    s = scenes.base_settings(slosh.settings_default, grid, 300000)
+    s.pcg_iterations, s.min_substeps, s.max_substeps, s.mg_smoothing_sweeps = 6, 1, 1, 2
+    s.gravity[:] = [0.0, 0.0, 0.0]
+    return s, scenes.fill_cells((10, 10, 10), (4, 4, 4)), scenes.fill_cells((48, 16, 8), (40, 48, 16))
+
+
+# A tank that is filled after a frame with few bricks is not solved by the few CTAs that those chose, however it is filled.
+@pytest.mark.parametrize("how", ["frame", "emit", "upload", "write"])
+def test_a_filled_tank_leaves_the_cluster(slosh, how):
+    s, drop, block = _drop_and_block(slosh)
+    full = slosh.Simulation(s)
+    full.step_frame(A.frame_input(s, emits=[drop, block]))
+    records = full.particles()
+    g = slosh.Simulation(s)
+    g.step_frame(A.frame_input(s, emits=[drop]))
+    assert _launches(g, A.frame_input(s)) < 50
+    if how == "emit":
+        g.emit(block)
+    elif how == "upload":
+        g.upload_particles(records)
+    elif how == "write":
+        g.write("PARTICLES", records)
+        g.write("BRICK_TOUCH", full.read("BRICK_TOUCH"))
+    n = _launches(g, A.frame_input(s, emits=[block] if how == "frame" else []))
+    assert int(g.read("ACTIVE_BRICKS")[0]) > 240 and n > 90, n
+
+
+# An emitter that feeds the tank every frame, wherever it started, does not leave it.
+@pytest.mark.parametrize("count", [40, 41])
+def test_a_steady_emitter_keeps_the_cluster(slosh, count):
+    s, drop, _ = _drop_and_block(slosh)
+    e = A.EmitRequest()
+    e.shape, e.count = A.EMIT_SPHERE, 40
+    e.center[:] = [48 * s.cell_size, 48 * s.cell_size, 32 * s.cell_size]
+    e.extent[:] = [14 * s.cell_size, 0.0, 0.0]  # 6^3 bricks with the layer around them
+    e.rotation[:] = [0.0, 0.0, 0.0, 1.0]
+    g = slosh.Simulation(s)
+    g.step_frame(A.frame_input(s, emits=[drop, e]))
+    for f in range(3):
+        e.count = 40 if f == 0 else count
+        assert _launches(g, A.frame_input(s, emits=[e])) < 50, f
+    n = int(g.read("ACTIVE_BRICKS")[0])
+    assert n + n // 16 <= 240  # what a cluster takes
