@@ -922,7 +922,7 @@ struct Ctx {
             if (P.viscosity_alpha > 0.0f && S.viscosity_iterations > 0) {
                 // the words lie in the solver's q, which no solve uses now; the first iteration's source is the field itself
                 uint8_t* words = reinterpret_cast<uint8_t*>(mg.q);
-                count(launch_viscosity_words(d, words, shape, stream));
+                count(launch_viscosity_words(d, words, V[0], V[1], shape, stream));
                 int src = 1;
                 for (int it = 0; it < S.viscosity_iterations; ++it) {
                     const int dst = src == 1 ? 2 : 1;

@@ -45,8 +45,9 @@ int launch_clear_new_slots(const Dev& d, const Shape& sh, cudaStream_t s);
 // ---- grid passes ----
 int launch_mark_cells(const Dev& d, const Pass& p, const Shape& sh, cudaStream_t s);
 int launch_normalize_faces(const Dev& d, const Pass& p, float* vel, const Shape& sh, cudaStream_t s);
-// One Jacobi iteration of the viscosity; words: 3 x pool_cells bytes, built once per substep from the face flags.
-int launch_viscosity_words(const Dev& d, uint8_t* words, const Shape& sh, cudaStream_t s);
+// One Jacobi iteration of the viscosity; words: 3 x pool_cells bytes, built once per substep from the face flags, by a pass that
+// also copies the field to the iterations' second buffer.
+int launch_viscosity_words(const Dev& d, uint8_t* words, const float* vel, float* copy, const Shape& sh, cudaStream_t s);
 int launch_viscosity(const Dev& d, const Pass& p, const uint8_t* words, const float* ustar, const float* src, float* dst, const Shape& sh,
                      cudaStream_t s);
 int launch_divergence(const Dev& d, const Pass& p, const float* vel, const Shape& sh, cudaStream_t s);

@@ -392,7 +392,11 @@ __global__ void __launch_bounds__(GRID_THREADS) k_normalize(Dev d, Pass p, float
 // face's values and its six neighbours' in one round, where it read the flags and each neighbour's flag before its value: the
 // grid phase of a 96x96x72 substep with 12 iterations (16.1 us each) took 239 us, 111 now.
 constexpr uint32_t VISC_MOVES = 1u << 6;
-__global__ void __launch_bounds__(GRID_THREADS) k_viscosity_words(Dev d, uint8_t* __restrict__ words) {
+// The copy of the field is what the buffer keeps where no iteration writes: a brick's cells outside the grid and free slots,
+// which the velocity buffers show to a caller (as a copy of its own before this pass it took 10 us of such a frame).
+__global__ void __launch_bounds__(GRID_THREADS) k_viscosity_words(Dev d, uint8_t* __restrict__ words, const float4* __restrict__ vel,
+                                                                  float4* __restrict__ copy) {
+    for (uint32_t i = blockIdx.x * GRID_THREADS + threadIdx.x; i < d.total_faces / 4u; i += gridDim.x * GRID_THREADS) copy[i] = vel[i];
     for_active_cells<true>(d, [&](uint32_t index, int3 c) {
         uint32_t own[3], nf[3][6];
 #pragma unroll
@@ -897,8 +901,8 @@ int launch_normalize_faces(const Dev& d, const Pass& p, float* vel, const Shape&
     k_normalize<<<sh.brick_ctas, GRID_THREADS, 0, s>>>(d, p, vel);
     return 1;
 }
-int launch_viscosity_words(const Dev& d, uint8_t* words, const Shape& sh, cudaStream_t s) {
-    k_viscosity_words<<<sh.brick_ctas, GRID_THREADS, 0, s>>>(d, words);
+int launch_viscosity_words(const Dev& d, uint8_t* words, const float* vel, float* copy, const Shape& sh, cudaStream_t s) {
+    k_viscosity_words<<<sh.brick_ctas, GRID_THREADS, 0, s>>>(d, words, reinterpret_cast<const float4*>(vel), reinterpret_cast<float4*>(copy));
     return 1;
 }
 int launch_viscosity(const Dev& d, const Pass& p, const uint8_t* words, const float* ustar, const float* src, float* dst, const Shape& sh,
