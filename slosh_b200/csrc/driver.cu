@@ -172,11 +172,9 @@ struct Ctx {
     SortBuffers sortb{};
     P2GGather gather{};  // the per-cell particle index of the gather P2G (allocated only when it is on)
     MGState mg{};
-    // Most CTAs of the solve's cluster form for this layout (0: not available, -1: not asked yet). The question loads two
-    // kernels and takes 3 ms of about 30 of a context's creation, so a layout of more bricks than this asks when its tank
-    // first has few enough active ones.
-    static constexpr uint32_t CLUSTER_LAYOUT = 2048;
-    int cluster_most = 0;
+    // Most CTAs of the solve's cluster form for this layout (0: not available, -1: not asked yet). Asked by the first solve that
+    // is small enough: the question loads the solver's device code, which a context that builds surfaces or sorts never needs.
+    int cluster_most = -1;
     // What the host knows of the active bricks (expected_bricks): the last stepped frame's most, or the layout's before the first
     // one and after records or state were written from outside; and the bricks that emissions since then can wake.
     uint32_t bricks_last = 0;
@@ -479,7 +477,7 @@ struct Ctx {
         prev_dt = 0.0f;
         last_max_speed = 0.0f;
         forget_bricks();
-        cluster_most = bricks_last <= CLUSTER_LAYOUT ? mg_solve_clusters(mg) : -1;
+        cluster_most = -1;
         shape.num_sms = num_sms;
         shape.brick_ctas = brick_ctas_for(ctas_per_sm);
         shape.mg_ctas = brick_ctas_for(mg_ctas_per_sm);

@@ -2547,8 +2547,7 @@ int mid_level(const MGState& m, int tail) {
 
 // The largest cluster that the solve of this hierarchy can run with on the current device: 16 CTAs, or 8 where no 16 can be
 // placed together, or 0 (a single level, a tail that starts below level 3, an alternative form asked for by the environment, no
-// room). Smaller clusters of the same CTAs fit wherever a larger one does. (An occupancy query takes milliseconds, so one
-// kernel and size is asked.)
+// room). Smaller clusters of the same CTAs fit wherever a larger one does.
 // A cell of level 4 has children in several bricks, so grids of more than 4,096 level-3 cells (136^3) have no resident form; their
 // few active bricks in the streamed one, on 4 to 16 SMs, took longer than launches over the whole GPU (a frame of 256^3 cells:
 // 39 bricks 1,032 against 939 us, 128 bricks with two sweep pairs 1,502 against 1,251).
