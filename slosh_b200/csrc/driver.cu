@@ -784,7 +784,10 @@ struct Ctx {
         // few active bricks: the whole solve in one cluster (the form does not change the result, so what the host knows is
         // enough to choose by)
         const uint32_t bricks = expected_bricks();
-        if (cluster_most < 0 && mg_solve_cluster(16, bricks) > 0) cluster_most = mg_solve_clusters(mg);
+        if (cluster_most < 0 && mg_solve_cluster(16, bricks) > 0) {
+            CK(cudaGetLastError());  // of the substep's launches so far: the question clears its own errors
+            cluster_most = mg_solve_clusters(mg);
+        }
         const int cluster = mg_solve_cluster(cluster_most, bricks);
         SolveGraph* G = nullptr;
         if (use_graphs && cluster == 0) {

@@ -2556,18 +2556,22 @@ int mg_solve_clusters(const MGState& m) {
     if (m.num_levels < 2 || tail > 3 || mg_staged() || mid_level(m, tail) > 0) return 0;
     const size_t smem = cl_smem(m);
     if (smem > size_t(CL_MAX_SMEM)) return 0;
-    bool ok = true;
+    // an error of these calls is an answer (no cluster) and is cleared; the caller has collected those of earlier launches
+    auto fine = [](cudaError_t e) {
+        if (e != cudaSuccess) cudaGetLastError();
+        return e == cudaSuccess;
+    };
     for (auto kernel : {k_solve_cluster<false>, k_solve_cluster<true>})
-        ok = ok && cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-             cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CL_MAX_SMEM) == cudaSuccess;
+        if (!fine(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) ||
+            !fine(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CL_MAX_SMEM)))
+            return 0;
     for (int ctas : {16, 8}) {
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute attr[1];
         cl_config(cfg, attr, ctas, smem, nullptr);
         int clusters = 0;
-        if (ok && cudaOccupancyMaxActiveClusters(&clusters, k_solve_cluster<true>, &cfg) == cudaSuccess && clusters > 0) return ctas;
+        if (fine(cudaOccupancyMaxActiveClusters(&clusters, k_solve_cluster<true>, &cfg)) && clusters > 0) return ctas;
     }
-    cudaGetLastError();
     return 0;
 }
 // The cluster for a tank of about `bricks` active bricks: the smallest whose resident form holds them with a sixteenth to
