@@ -5,7 +5,7 @@ import pytest
 from slosh_b200 import _abi as A
 from slosh_b200 import scenes
 
-from parity import pair, run_frames
+from parity import compare_state, pair, run_frames
 
 pytestmark = pytest.mark.gpu
 
@@ -127,3 +127,39 @@ def test_a_steady_emitter_keeps_the_cluster(slosh, count):
         assert _launches(g, A.frame_input(s, emits=[e])) < 50, f
     n = int(g.read("ACTIVE_BRICKS")[0])
     assert n + n // 16 <= 240  # what a cluster takes
+
+
+# A tank that outgrows its cluster within a frame: a spray crosses brick boundaries, the cluster was chosen by the frame before,
+# and the solve goes on over global memory. Tails at levels 1 to 3, several options each.
+@pytest.mark.parametrize("grid,cells", [((32, 32, 32), 6), ((64, 64, 64), 14), ((104, 96, 100), 14)])
+@pytest.mark.parametrize("settings", [
+    dict(tolerance=0.0, pcg_iterations=3),
+    dict(tolerance=1e-6, mg_smoothing_sweeps=2, mg_correction_scale=1.9, mg_coarse_iterations=4, mg_smoother_weight=1.15),
+    dict(tolerance=1e-5, precision_mode=A.PRECISION_BF16_STORAGE, pcg_flexible=1, mg_smoothing_sweeps=3),
+    dict(tolerance=1e-5, precision_mode=A.PRECISION_FP16_STORAGE, pcg_flexible=1, mg_smoother_weight=1.15),
+])
+def test_growth_within_a_frame_matches_oracle(slosh, oracle_mod, grid, cells, settings):
+    s = scenes.base_settings(slosh.settings_default, grid, 8 * cells ** 3)
+    s.cell_size = 1.0 / max(grid)
+    s.max_frame_dt = 1.0 / 30.0
+    for k, v in settings.items():
+        setattr(s, k, v)
+    e = scenes.fill_cells((9, 9, 9), (cells, cells, cells), velocity=tuple([5.0 * 60.0 * s.cell_size] * 3))  # 5 cells in a sixtieth
+    e.velocity_spread, e.speed_jitter = 0.2, 0.4
+    g, o = slosh.Simulation(s), oracle_mod.Oracle(s)
+    bricks = []
+    for f in range(3):
+        s.min_substeps = s.max_substeps = 1 if f < 2 else 6
+        fi = A.frame_input(s, emits=[e] if f == 0 else [], delta_time=1e-4 if f < 2 else 1.0 / 60.0)
+        assert g.begin_frame(fi) == o.begin_frame(fi)
+        for k in range(1 if f < 2 else 6):
+            g.substep(k)
+            o.substep(k)
+            bad = compare_state(g, o).failures()
+            assert not bad, (f, k, bad)
+            bricks.append(int(g.read("ACTIVE_BRICKS")[0]))
+        g.end_frame()
+        o.end_frame()
+        assert g.results().last_solve_iterations == o.results().last_solve_iterations
+    ctas = next(c for c in range(4, 18, 2) if bricks[1] + bricks[1] // 16 <= 16 * (c - 1))
+    assert ctas <= 16 and bricks[-1] > 16 * (ctas - 1), bricks
