@@ -435,8 +435,8 @@ __device__ __forceinline__ void w0_black(const Dev& d, const MGState& m, Prep pr
 // cell order, 5.0 so (a frame of 200 + 30 iterations 11.8 -> 3.45 -> 2.96 ms; four rounds' loads in flight need a second
 // wave of CTAs: 3.7 ms).
 // PARTS = 4: a quarter of a brick per warp, one round of loads instead of two, while all of the quarters are resident
-// (RB_SMALL_BRICKS): a frame of a 96x96x72 tank 1.19 -> 1.06 ms (half a brick 1.11); the large one 2.96 -> 3.76 ms.
-constexpr uint32_t RB_SMALL_BRICKS = 1480;  // their quarters are 148 SMs x RB_SMALL_CTAS x 8 warps
+// (RB_SMALL_CTAS a SM: 1,480 bricks on 148 SMs): a frame of a 96x96x72 tank 1.19 -> 1.06 ms (half a brick 1.11); the large one
+// 2.96 -> 3.76 ms.
 constexpr int RB_SMALL_CTAS = 5;
 // Entry 2 t + 64 k of lane t in round k, its row y and plane z, and whether its red cells lie at odd x.
 struct RbGeo {
@@ -2799,7 +2799,7 @@ int launch_rbgs(const Dev& d, const MGState& m, float* pres, const float* rhs, i
                 cudaStream_t s) {
     if (first) launch_k(k_pcg_words, sh.mg_ctas, GRID_THREADS, 0, s, d, m);
     launch_k(first ? k_rbgs_split<true> : k_rbgs_split<false>, sh.mg_ctas, GRID_THREADS, 0, s, d, m, pres, rhs);
-    const bool small = bricks <= RB_SMALL_BRICKS;
+    const bool small = 4u * bricks <= uint32_t(sh.num_sms * RB_SMALL_CTAS * (GRID_THREADS / 32));
     for (int it = 0; it < sweeps; ++it)
         for (uint32_t colour = 0; colour < 2u; ++colour)
             launch_k(small ? k_rbgs<4> : k_rbgs<1>, small ? sh.num_sms * RB_SMALL_CTAS : sh.mg_ctas, GRID_THREADS, 0, s, d, m, colour, omega);
