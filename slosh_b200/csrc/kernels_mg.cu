@@ -1144,7 +1144,13 @@ __global__ void k_prolong_smooth_fp(Dev d, MGState m, int l) {
 // 1,024 tiles) 1,876 -> 1,608, of 128x128x96 substeps with one sweep pair (from level 2) 815 -> 784 a frame. With 256 threads and
 // 4 loads in flight slower than the launches (2,603 us); level 1 of 256^3 (4,096 tiles, most of them empty) too (2,567 us, 2,297
 // with a list of the tiles that hold active bricks).
-constexpr int CT_SIDE = 8, CT_THREADS = 1024, CT_LEVEL1_TILES = 1536;
+// Levels are fused from the first one of at most CT_TILES tiles per SM on, four waves of two CTAs. Frames with two sweep pairs, level 1
+// launched and fused, of a tank with little, some and much liquid: 1,000 tiles (160^3) 1,216 and 1,181, 2,354 and 2,352, 5,164 and
+// 5,125 us; 1,024 (256x128x128) 1,139 and 1,088, 2,270 and 2,261, 4,709 and 4,719; 1,331 (176^3) 1,156 and 1,152, 2,615 and 2,668, 6,170 and
+// 6,318; 1,728 (192^3) 1,223 and 1,227, 2,763 and 2,811, 7,296 and 7,460; 4,096 (256^3) 1,350 and 1,601, 4,948 and 5,449. With one
+// sweep pair, level 2 launched and fused, little and much liquid: 1,000 (320^3) 1,097 and 1,098, 2,513 and 2,363; 2,197 (400^3) 1,094 and
+// 1,263, 3,672 and 3,852; 4,096 (512^3) 1,178 and 1,541, 6,820 and 7,230. The count decides, hardly the share of empty tiles.
+constexpr int CT_SIDE = 8, CT_THREADS = 1024, CT_TILES = 8;
 template <int S> struct CoarseTile {
     static constexpr int H = 2 * S, R = CT_SIDE + 2 * H, CELLS = R * R * R;
     float x[CELLS], b[CELLS];
@@ -2721,9 +2727,10 @@ int launch_vcycle(const Dev& d, const MGState& m, int coarse_iterations, const S
         const int3 t = ct_tiles(m.lv[l]);
         return t.x * t.y * t.z;
     };
-    // levels from here to the tail run one fused pass each way: level 2 up, and level 1 where two sweep pairs leave it the
-    // most launches and its tiles are few (mostly empty tiles and the halo's work cost more than launches beyond that)
-    const int fused = mid > 0 || sweeps > 2 ? tail : (sweeps == 2 && tiles(1) <= CT_LEVEL1_TILES ? 1 : 2);
+    // levels from here to the tail run one fused pass each way: level 2 up, and level 1 where two sweep pairs leave it the most
+    // launches, without levels of many tiles (their tests, loads and halos cost more than the launches)
+    int fused = mid > 0 || sweeps > 2 ? tail : (sweeps == 2 ? 1 : 2);
+    while (fused < tail && tiles(fused) > CT_TILES * sh.num_sms) ++fused;
     for (int l = 0; l < down_end; ++l) {
         if (l >= fused) {
             if (sweeps == 1) launch_k(k_coarse_down<1>, tiles(l), CT_THREADS, 0, s, m, l);

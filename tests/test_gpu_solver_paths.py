@@ -163,3 +163,22 @@ def test_growth_within_a_frame_matches_oracle(slosh, oracle_mod, grid, cells, se
         assert g.results().last_solve_iterations == o.results().last_solve_iterations
     ctas = next(c for c in range(4, 18, 2) if bricks[1] + bricks[1] // 16 <= 16 * (c - 1))
     assert ctas <= 16 and bricks[-1] > 16 * (ctas - 1), bricks
+
+
+# levels 1 and 2 have too many tiles for the fused coarse passes, levels 3 and 4 do not
+@pytest.mark.parametrize("settings", [
+    dict(pcg_iterations=3),
+    dict(pcg_iterations=3, mg_smoothing_sweeps=2, mg_correction_scale=1.9, mg_smoother_weight=1.15),
+    dict(pcg_iterations=2, mg_smoothing_sweeps=2, precision_mode=A.PRECISION_BF16_STORAGE, pcg_flexible=1),
+])
+def test_fused_levels_below_launched_ones_match_oracle(slosh, oracle_mod, settings):
+    grid = (97, 129, 2048)
+    s = scenes.base_settings(slosh.settings_default, grid, 150000)
+    s.cell_size = 1.0 / 64.0
+    s.sparse_storage_budget = 0.05
+    s.min_substeps = s.max_substeps = 1
+    for k, v in settings.items():
+        setattr(s, k, v)
+    sc = dict(settings=s, emits=[scenes.fill_cells((30, 40, 1000), (24, 24, 30))], seed=1)
+    g, o = pair(slosh, oracle_mod, sc)
+    run_frames(g, o, sc, frames=2, tol=None)
