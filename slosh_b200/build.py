@@ -12,7 +12,7 @@ BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libslosh_b200.so")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 SOURCES = ["driver.cu", "kernels_grid.cu", "kernels_particles.cu", "kernels_mg.cu", "kernels_sort.cu", "sort_static.cu", "kernels_surface.cu", "kernels_unet.cu", "unet.cu"]
-HEADERS = ["common.cuh", "g2p_box.h", "kernels.h", "mg_cluster.cuh", "splat_box.h", "tc.cuh", "unet.h"]
+HEADERS = ["common.cuh", "exact_div.h", "g2p_box.h", "kernels.h", "mg_cluster.cuh", "splat_box.h", "tc.cuh", "unet.h"]
 # The device code is not compressed: the solver's (12 MB, most of it line tables) took 12 ms to unpack at its first use in a
 # process, 5 as it is.
 FLAGS = [

@@ -26,6 +26,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include "exact_div.h"
 #include "kernels.h"
 #include "tc.cuh"
 
@@ -560,17 +561,6 @@ __global__ void __launch_bounds__(GRID_THREADS) k_rbgs(Dev d, MGState m, uint32_
     }
 }
 
-// a / d correctly rounded, rc = the correctly rounded 1 / d (Markstein's theorem, IBM J. Res. Dev. 34 (1), 1990: a
-// faithful quotient corrected once by its exact remainder times rc is the rounded quotient; the first correction makes
-// the product faithful). Five dependent operations where the division takes about 200 cycles. The remainders are exact
-// only away from the ends of the exponent range: outside [1e-25, 1e25] the division itself.
-__device__ __forceinline__ float div_by(float a, float d, float rc) {
-    const float m = fabsf(a);
-    if (!(m >= 1e-25f && m <= 1e25f)) return a == 0.0f ? a * rc : a / d;
-    float q = a * rc;
-    q = __fmaf_rn(__fmaf_rn(-q, d, a), rc, q);
-    return __fmaf_rn(__fmaf_rn(-q, d, a), rc, q);
-}
 struct Nb6 {
     uint32_t w;
     float c0, c1, c2;
