@@ -799,158 +799,154 @@ __device__ __forceinline__ void g2p_particle(const Dev& d, const Pass& p, slosh_
         return make_float3(rb.x, rb.y, rb.z);
     };
     if (p.use_apic == 0u) P.vel = old_vel();
-    {
-        {
-            const float h = d.h, inv_h = d.inv_h, dt = p.dt;
-            const float lo = h * 1.01f;
-            const float3 hi = make_float3((float(d.grid.x) - 1.01f) * h, (float(d.grid.y) - 1.01f) * h, (float(d.grid.z) - 1.01f) * h);
-            float3 pic, delta, dw, gx, gy, gz;
-            const uint32_t zero_c = pack_half2(0.0f, 0.0f);
-            uint32_t cw[5] = {zero_c, zero_c, zero_c, zero_c, zero_c};  // the packed APIC rows (zero for PIC/FLIP)
-            float3 grad[3];
-            field.gather(d, p, P.pos, pic, delta, dw, grad);
-            gx = grad[0]; gy = grad[1]; gz = grad[2];
-            float3 nv;
-            if (p.use_apic) {
-                nv = pic;
-                // the new rows packed to halves at once: 5 words live to the store instead of 9 floats
-                cw[0] = pack_half2(gx.x, gx.y);
-                cw[1] = pack_half2(gx.z, gy.x);
-                cw[2] = pack_half2(gy.y, gy.z);
-                cw[3] = pack_half2(gz.x, gz.y);
-                cw[4] = pack_half2(gz.z, 0.0f);
-            } else {
-                const float fdx = dw.x > 1e-4f ? delta.x / dw.x : pic.x - P.vel.x;
-                const float fdy = dw.y > 1e-4f ? delta.y / dw.y : pic.y - P.vel.y;
-                const float fdz = dw.z > 1e-4f ? delta.z / dw.z : pic.z - P.vel.z;
-                const float3 target = make_float3(P.vel.x + fdx, P.vel.y + fdy, P.vel.z + fdz);
-                nv = make_float3(pic.x + p.flip_ratio * (target.x - pic.x), pic.y + p.flip_ratio * (target.y - pic.y),
-                                 pic.z + p.flip_ratio * (target.z - pic.z));
-            }
-            // RK2 midpoint with the Euler blend.
-            const float3 v1 = pic;
-            const float half_dt = 0.5f * dt;
-            float3 mid = addf3(P.pos, scale3(half_dt, v1));
-            mid = make_float3(clampf(mid.x, lo, hi.x), clampf(mid.y, lo, hi.y), clampf(mid.z, lo, hi.z));
-            const float mid_cells = half_dt * len3(v1) * inv_h;
-            float3 v2 = v1;
-            if (mid_cells < 2.0f) {
-                const bool check = mid_cells > 1.0f;
-                const float3 sv = field.sample(d, mid, v1, check);
-                const float t = saturatef(mid_cells - 1.0f);
-                v2 = make_float3(sv.x + t * (v1.x - sv.x), sv.y + t * (v1.y - sv.y), sv.z + t * (v1.z - sv.z));
-            }
-            float3 x = addf3(P.pos, scale3(dt, v2));
-            if (apply_density) {
-                const float3 cpos = make_float3(clampf(P.pos.x, lo, hi.x), clampf(P.pos.y, lo, hi.y), clampf(P.pos.z, lo, hi.z));
-                x = addf3(x, field.displacement(d, cpos));
-            }
-            // Pool exhausted: ballistic.
-            const int3 pcell = make_int3(clampi(int(floorf(P.pos.x * inv_h)), 0, d.grid.x - 1),
-                                         clampi(int(floorf(P.pos.y * inv_h)), 0, d.grid.y - 1),
-                                         clampi(int(floorf(P.pos.z * inv_h)), 0, d.grid.z - 1));
-            if (is_null_cell(cell_index(d, pcell))) {
-                const float3 g = make_float3(p.gravity[0], p.gravity[1], p.gravity[2]);
-                nv = addf3(old_vel(), mul3s(g, dt));
-                x = addf3(P.pos, scale3(dt, nv));
+    const float h = d.h, inv_h = d.inv_h, dt = p.dt;
+    const float lo = h * 1.01f;
+    const float3 hi = make_float3((float(d.grid.x) - 1.01f) * h, (float(d.grid.y) - 1.01f) * h, (float(d.grid.z) - 1.01f) * h);
+    float3 pic, delta, dw, gx, gy, gz;
+    const uint32_t zero_c = pack_half2(0.0f, 0.0f);
+    uint32_t cw[5] = {zero_c, zero_c, zero_c, zero_c, zero_c};  // the packed APIC rows (zero for PIC/FLIP)
+    float3 grad[3];
+    field.gather(d, p, P.pos, pic, delta, dw, grad);
+    gx = grad[0]; gy = grad[1]; gz = grad[2];
+    float3 nv;
+    if (p.use_apic) {
+        nv = pic;
+        // the new rows packed to halves at once: 5 words live to the store instead of 9 floats
+        cw[0] = pack_half2(gx.x, gx.y);
+        cw[1] = pack_half2(gx.z, gy.x);
+        cw[2] = pack_half2(gy.y, gy.z);
+        cw[3] = pack_half2(gz.x, gz.y);
+        cw[4] = pack_half2(gz.z, 0.0f);
+    } else {
+        const float fdx = dw.x > 1e-4f ? delta.x / dw.x : pic.x - P.vel.x;
+        const float fdy = dw.y > 1e-4f ? delta.y / dw.y : pic.y - P.vel.y;
+        const float fdz = dw.z > 1e-4f ? delta.z / dw.z : pic.z - P.vel.z;
+        const float3 target = make_float3(P.vel.x + fdx, P.vel.y + fdy, P.vel.z + fdz);
+        nv = make_float3(pic.x + p.flip_ratio * (target.x - pic.x), pic.y + p.flip_ratio * (target.y - pic.y),
+                         pic.z + p.flip_ratio * (target.z - pic.z));
+    }
+    // RK2 midpoint with the Euler blend.
+    const float3 v1 = pic;
+    const float half_dt = 0.5f * dt;
+    float3 mid = addf3(P.pos, scale3(half_dt, v1));
+    mid = make_float3(clampf(mid.x, lo, hi.x), clampf(mid.y, lo, hi.y), clampf(mid.z, lo, hi.z));
+    const float mid_cells = half_dt * len3(v1) * inv_h;
+    float3 v2 = v1;
+    if (mid_cells < 2.0f) {
+        const bool check = mid_cells > 1.0f;
+        const float3 sv = field.sample(d, mid, v1, check);
+        const float t = saturatef(mid_cells - 1.0f);
+        v2 = make_float3(sv.x + t * (v1.x - sv.x), sv.y + t * (v1.y - sv.y), sv.z + t * (v1.z - sv.z));
+    }
+    float3 x = addf3(P.pos, scale3(dt, v2));
+    if (apply_density) {
+        const float3 cpos = make_float3(clampf(P.pos.x, lo, hi.x), clampf(P.pos.y, lo, hi.y), clampf(P.pos.z, lo, hi.z));
+        x = addf3(x, field.displacement(d, cpos));
+    }
+    // Pool exhausted: ballistic.
+    const int3 pcell = make_int3(clampi(int(floorf(P.pos.x * inv_h)), 0, d.grid.x - 1),
+                                 clampi(int(floorf(P.pos.y * inv_h)), 0, d.grid.y - 1),
+                                 clampi(int(floorf(P.pos.z * inv_h)), 0, d.grid.z - 1));
+    if (is_null_cell(cell_index(d, pcell))) {
+        const float3 g = make_float3(p.gravity[0], p.gravity[1], p.gravity[2]);
+        nv = addf3(old_vel(), mul3s(g, dt));
+        x = addf3(P.pos, scale3(dt, nv));
 #pragma unroll
-                for (int k = 0; k < 5; ++k) cw[k] = zero_c;
+        for (int k = 0; k < 5; ++k) cw[k] = zero_c;
+    }
+    // Force-field manipulators.
+    for (uint32_t m = 0; m < p.num_manipulators; ++m) {
+        const slosh_manipulator_t& f = d.manipulators[m];
+        if (f.kind == MANIP_DRAIN) continue;
+        const float w = manipulator_weight(f, x);
+        if (w <= 0.0f) continue;
+        const float3 r = sub3(x, ld3(f.center));
+        const float3 ax = ld3(f.axis);
+        if (f.kind == MANIP_DIRECTIONAL) {
+            nv = addf3(nv, mul3s(ax, f.strength * w * dt));
+        } else if (f.kind == MANIP_RADIAL) {
+            const float rl = len3(r);
+            const float3 nn = rl > 1e-5f ? make_float3(r.x / rl, r.y / rl, r.z / rl) : make_float3(0.0f, 0.0f, 0.0f);
+            nv = addf3(nv, mul3s(nn, f.strength * w * dt));
+        } else if (f.kind == MANIP_SWIRL) {
+            const float3 perp = sub3(r, scale3(dot3(r, ax), ax));
+            const float pl = len3(perp);
+            if (pl > 1e-5f) {
+                const float3 pn = make_float3(perp.x / pl, perp.y / pl, perp.z / pl);
+                const float3 tangent = cross3(ax, pn);
+                nv = addf3(nv, mul3s(sub3(tangent, mul3s(pn, f.param0)), f.strength * w * dt));
             }
-            // Force-field manipulators.
-            for (uint32_t m = 0; m < p.num_manipulators; ++m) {
-                const slosh_manipulator_t& f = d.manipulators[m];
-                if (f.kind == MANIP_DRAIN) continue;
-                const float w = manipulator_weight(f, x);
-                if (w <= 0.0f) continue;
-                const float3 r = sub3(x, ld3(f.center));
-                const float3 ax = ld3(f.axis);
-                if (f.kind == MANIP_DIRECTIONAL) {
-                    nv = addf3(nv, mul3s(ax, f.strength * w * dt));
-                } else if (f.kind == MANIP_RADIAL) {
-                    const float rl = len3(r);
-                    const float3 nn = rl > 1e-5f ? make_float3(r.x / rl, r.y / rl, r.z / rl) : make_float3(0.0f, 0.0f, 0.0f);
-                    nv = addf3(nv, mul3s(nn, f.strength * w * dt));
-                } else if (f.kind == MANIP_SWIRL) {
-                    const float3 perp = sub3(r, scale3(dot3(r, ax), ax));
-                    const float pl = len3(perp);
-                    if (pl > 1e-5f) {
-                        const float3 pn = make_float3(perp.x / pl, perp.y / pl, perp.z / pl);
-                        const float3 tangent = cross3(ax, pn);
-                        nv = addf3(nv, mul3s(sub3(tangent, mul3s(pn, f.param0)), f.strength * w * dt));
-                    }
-                } else if (f.kind == MANIP_DRAG) {
-                    nv = mul3s(nv, exp_r(-f.strength * w * dt));
-                }
-            }
-            // Colliders.
-            const float radius = p.particle_radius, adh = p.adhesion_accel, adh_range = p.adhesion_range, friction = p.friction;
-            for (uint32_t k = 0; k < p.num_colliders; ++k) {
-                const slosh_collider_t& c = d.colliders[k];
-                const float dist = collider_sdf(c, x);
-                if (adh > 0.0f && dist < radius + adh_range) {
-                    const float3 nn = collider_normal(c, x, 0.25f * h);
-                    const float w = saturatef(1.0f - (dist - radius) / adh_range);
-                    const float3 vs = collider_velocity_at(c, x);
-                    const float vn = dot3(sub3(nv, vs), nn);
-                    nv = sub3(nv, mul3s(nn, fminf(adh * w * dt, fmaxf(vn, 0.0f) + adh * w * dt * 0.25f)));
-                }
-                if (dist < radius) {
-                    const float3 nn = collider_normal(c, x, 0.25f * h);
-                    x = addf3(x, mul3s(nn, radius - dist));
-                    const float3 vs = collider_velocity_at(c, x);
-                    float3 rel = sub3(nv, vs);
-                    const float vn = dot3(rel, nn);
-                    if (vn < 0.0f) {
-                        rel = sub3(rel, scale3(vn, nn));
-                        rel = sub3(rel, scale3(friction, sub3(rel, scale3(dot3(rel, nn), nn))));
-                    }
-                    nv = addf3(vs, rel);
-                }
-            }
-            // Domain walls.
-            uint32_t wall = 0u;
-            float xs[3] = {x.x, x.y, x.z}, vs[3] = {nv.x, nv.y, nv.z};
-            const float his[3] = {hi.x, hi.y, hi.z};
-#pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                if (xs[a] < lo) { xs[a] = lo; vs[a] = fmaxf(vs[a], 0.0f); wall |= 1u << a; }
-                else if (xs[a] > his[a]) { xs[a] = his[a]; vs[a] = fminf(vs[a], 0.0f); wall |= 1u << a; }
-            }
-            if (wall != 0u && friction > 0.0f) {
-#pragma unroll
-                for (int a = 0; a < 3; ++a)
-                    if ((wall & (1u << a)) == 0u) vs[a] = vs[a] * (1.0f - friction);
-            }
-            x = make_float3(xs[0], xs[1], xs[2]);
-            nv = make_float3(vs[0], vs[1], vs[2]);
-            const float speed = len3(nv);
-            if (speed > p.max_speed) {
-                atomicAdd(d.stats + 9, 1u);
-                atomicAdd(d.stats + 10, __float2uint_rz(x.x * 100.0f));
-                atomicAdd(d.stats + 11, __float2uint_rz(x.y * 100.0f));
-                atomicAdd(d.stats + 12, __float2uint_rz(x.z * 100.0f));
-                const int3 sc = make_int3(int(floorf(P.pos.x * inv_h)), int(floorf(P.pos.y * inv_h)), int(floorf(P.pos.z * inv_h)));
-                if (type_of(get_cell_type(d, sc)) == CELL_SOLID) atomicAdd(d.stats + 13, 1u);
-            }
-            bool drained = false;
-            for (uint32_t dr = 0; dr < p.num_manipulators && !drained; ++dr) {
-                const slosh_manipulator_t& f = d.manipulators[dr];
-                if (f.kind != MANIP_DRAIN || manipulator_sdf(f, x) > 0.0f) continue;
-                const float chance = f.param0 > 0.0f ? 1.0f - exp_r(-f.param0 * dt) : 1.0f;
-                if (chance >= 1.0f || hash_to_unit(pcg_hash(i * 2654435761u + p.frame_seed * 97u + dr)) < chance) {
-                    store_dead(particles, i);
-                    atomicAdd(d.stats + 15, 1u);
-                    drained = true;
-                }
-            }
-            if (!drained) {
-                g2p_store(particles, i, x, P.age + dt, nv, cw);
-                speed_bits = __float_as_uint(speed);
-                const int3 ec = make_int3(clampi(int(floorf(x.x * inv_h)), 0, d.grid.x - 1), clampi(int(floorf(x.y * inv_h)), 0, d.grid.y - 1),
-                                          clampi(int(floorf(x.z * inv_h)), 0, d.grid.z - 1));
-                brick = brick_index_of(d, make_int3(ec.x >> 3, ec.y >> 3, ec.z >> 3));
-            }
+        } else if (f.kind == MANIP_DRAG) {
+            nv = mul3s(nv, exp_r(-f.strength * w * dt));
         }
+    }
+    // Colliders.
+    const float radius = p.particle_radius, adh = p.adhesion_accel, adh_range = p.adhesion_range, friction = p.friction;
+    for (uint32_t k = 0; k < p.num_colliders; ++k) {
+        const slosh_collider_t& c = d.colliders[k];
+        const float dist = collider_sdf(c, x);
+        if (adh > 0.0f && dist < radius + adh_range) {
+            const float3 nn = collider_normal(c, x, 0.25f * h);
+            const float w = saturatef(1.0f - (dist - radius) / adh_range);
+            const float3 vs = collider_velocity_at(c, x);
+            const float vn = dot3(sub3(nv, vs), nn);
+            nv = sub3(nv, mul3s(nn, fminf(adh * w * dt, fmaxf(vn, 0.0f) + adh * w * dt * 0.25f)));
+        }
+        if (dist < radius) {
+            const float3 nn = collider_normal(c, x, 0.25f * h);
+            x = addf3(x, mul3s(nn, radius - dist));
+            const float3 vs = collider_velocity_at(c, x);
+            float3 rel = sub3(nv, vs);
+            const float vn = dot3(rel, nn);
+            if (vn < 0.0f) {
+                rel = sub3(rel, scale3(vn, nn));
+                rel = sub3(rel, scale3(friction, sub3(rel, scale3(dot3(rel, nn), nn))));
+            }
+            nv = addf3(vs, rel);
+        }
+    }
+    // Domain walls.
+    uint32_t wall = 0u;
+    float xs[3] = {x.x, x.y, x.z}, vs[3] = {nv.x, nv.y, nv.z};
+    const float his[3] = {hi.x, hi.y, hi.z};
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        if (xs[a] < lo) { xs[a] = lo; vs[a] = fmaxf(vs[a], 0.0f); wall |= 1u << a; }
+        else if (xs[a] > his[a]) { xs[a] = his[a]; vs[a] = fminf(vs[a], 0.0f); wall |= 1u << a; }
+    }
+    if (wall != 0u && friction > 0.0f) {
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+            if ((wall & (1u << a)) == 0u) vs[a] = vs[a] * (1.0f - friction);
+    }
+    x = make_float3(xs[0], xs[1], xs[2]);
+    nv = make_float3(vs[0], vs[1], vs[2]);
+    const float speed = len3(nv);
+    if (speed > p.max_speed) {
+        atomicAdd(d.stats + 9, 1u);
+        atomicAdd(d.stats + 10, __float2uint_rz(x.x * 100.0f));
+        atomicAdd(d.stats + 11, __float2uint_rz(x.y * 100.0f));
+        atomicAdd(d.stats + 12, __float2uint_rz(x.z * 100.0f));
+        const int3 sc = make_int3(int(floorf(P.pos.x * inv_h)), int(floorf(P.pos.y * inv_h)), int(floorf(P.pos.z * inv_h)));
+        if (type_of(get_cell_type(d, sc)) == CELL_SOLID) atomicAdd(d.stats + 13, 1u);
+    }
+    bool drained = false;
+    for (uint32_t dr = 0; dr < p.num_manipulators && !drained; ++dr) {
+        const slosh_manipulator_t& f = d.manipulators[dr];
+        if (f.kind != MANIP_DRAIN || manipulator_sdf(f, x) > 0.0f) continue;
+        const float chance = f.param0 > 0.0f ? 1.0f - exp_r(-f.param0 * dt) : 1.0f;
+        if (chance >= 1.0f || hash_to_unit(pcg_hash(i * 2654435761u + p.frame_seed * 97u + dr)) < chance) {
+            store_dead(particles, i);
+            atomicAdd(d.stats + 15, 1u);
+            drained = true;
+        }
+    }
+    if (!drained) {
+        g2p_store(particles, i, x, P.age + dt, nv, cw);
+        speed_bits = __float_as_uint(speed);
+        const int3 ec = make_int3(clampi(int(floorf(x.x * inv_h)), 0, d.grid.x - 1), clampi(int(floorf(x.y * inv_h)), 0, d.grid.y - 1),
+                                  clampi(int(floorf(x.z * inv_h)), 0, d.grid.z - 1));
+        brick = brick_index_of(d, make_int3(ec.x >> 3, ec.y >> 3, ec.z >> 3));
     }
 }
 // Ends a G2P CTA: touch flags and the fastest particle. Sorted particles mostly share bricks, so only the first lane of
@@ -962,8 +958,8 @@ __device__ __forceinline__ void g2p_finish(const Dev& d, uint32_t brick, uint32_
     if ((threadIdx.x & 31) == 0 && speed_bits) atomicMax(d.stats + 0, speed_bits);
 }
 
-// Stencils straight from the brick pool through the brick table (PIC/FLIP, whose sums also need each node's flags and old
-// velocity).
+// Stencils straight from the brick pool through the brick table: PIC/FLIP, whose sums also need each node's flags and old
+// velocity, and APIC while the particles are in placement order.
 template <int MINB>
 __global__ void __launch_bounds__(G2P_THREADS, MINB) k_g2p(Dev d, Pass p, slosh_particle_t* __restrict__ particles, uint32_t n,
                                                      const float* __restrict__ vel, const float* __restrict__ disp,
@@ -983,8 +979,8 @@ __global__ void __launch_bounds__(G2P_THREADS, MINB) k_g2p(Dev d, Pass p, slosh_
 // brick table and forms eight indices for each of a particle's six (with the displacement nine) stencils, 1,061 warp
 // instructions per 32 particles without it, 1,430 with it. The margin holds the stencils of the RK2 midpoint up to a step
 // of two cells; positions that leave the tile, and CTAs whose box does not fit, read the pool.
-// Bound by issue (about 60 %) and the phases' latency (box, fill, advect), so CTAs of 384 threads, three per SM at 64
-// registers: 20.6 M particles at 256^3 with the displacement 1,266 us from the pool, 909 now; 6.2 M in 256x128x128 455 and 346;
+// Bound by issue (68 % of the slots) and the phases' latency (box, fill, advect), so CTAs of 384 threads, three per SM at 56
+// registers without spills: 20.6 M particles at 256^3 with the displacement 1,266 us from the pool, 909 now; 6.2 M in 256x128x128 455 and 346;
 // 1.7 M in 128x128x96 101 and 82. 512 threads, two per SM: 1,021; 256, four: 967; 384, four (40 registers): 958. Only positions
 // and ages are read of the records (the old velocity is FLIP's).
 constexpr int G2P_TILE_THREADS = 384;
