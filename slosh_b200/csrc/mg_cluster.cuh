@@ -18,10 +18,10 @@
 // Streamed form (more bricks than that): the launched kernels' bodies over global memory between cluster barriers.
 // Both give the launched form's bits.
 //
-// Used while the resident form held the tank's active bricks in its last frame. What bounds a pass now is its chain of
+// Used while the resident form holds the bricks that the tank is expected to have (mg_solve_cluster). What bounds a pass now is its chain of
 // barrier (0.3-0.5 us), distributed-shared-memory copy and sweep, 1.5-3 us for level 0; the tail is 9 of 35 us of an iteration of
-// a 64x64x48 tank (150 active bricks), which took 70 us as launches: its frame 1,034 -> 695 us; 24 tanks of 70-288 active bricks
-// stepped together 36.7 -> 13.2 ms.
+// a 64x64x48 tank (150 active bricks), which took 70 us as launches: its frame 1,034 -> 690 us; 24 tanks of 70-288 active bricks
+// stepped together 36.0 -> 16.2 to 16.4 ms.
 #pragma once
 
 constexpr int CL_THREADS = 512;  // 128 registers; a spilled value would come from L2 after every barrier (its acquire empties the L1)
