@@ -178,6 +178,7 @@ struct Ctx {
     // What the host knows of the active bricks (expected_bricks): the last stepped frame's most, or the layout's before the first
     // one and after records or state were written from outside; and the bricks that emissions since then can wake.
     uint32_t bricks_last = 0;
+    double fluid_last = 0.0;  // the last stepped frame's fluid cells, a substep's mean
     struct Emitted {
         int lo[3], hi[3];          // the emissions' common box of bricks, with the layer around it that the pool keeps
         uint64_t count, bricks;    // particles; sum of the single emissions' bounds
@@ -690,6 +691,7 @@ struct Ctx {
     }
     void forget_bricks() {
         bricks_last = num_pool_bricks - 1u;
+        fluid_last = 0.0;
         emitted = emitted_before = Emitted{};
     }
     // About how many bricks the coming solves have (at most; tanks also grow by flowing). A steady emitter's box holds the bricks
@@ -974,7 +976,7 @@ struct Ctx {
         }
         {
             PhaseScope ps(this, 8);
-            count(launch_g2p(d, P, particles[pbuf], num_particles, V[c], V[(c + 2) % 3], density, unsorted, stream));
+            count(launch_g2p(d, P, particles[pbuf], num_particles, V[c], V[(c + 2) % 3], density, unsorted || double(num_particles) < G2P_SPARSE * fluid_last, stream));
         }
         // The field of logical buffer c becomes logical buffer 0 for the next substep.
         const int nm[3] = {vmap[c], vmap[(c + 1) % 3], vmap[(c + 2) % 3]};
@@ -1015,6 +1017,7 @@ void Ctx::end_frame_finish() {
     CK(cudaStreamSynchronize(stream));
     if (substeps > 0) {
         bricks_last = h_stats[7];
+        fluid_last = double(h_stats[1]) / substeps;
         emitted_before = emitted;
         emitted = Emitted{};
         float ms;

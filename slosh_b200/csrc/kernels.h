@@ -69,8 +69,10 @@ int launch_emit(const Dev& d, slosh_particle_t* particles, const uint32_t* parti
 int launch_touch_particles(const Dev& d, const slosh_particle_t* particles, uint32_t n, cudaStream_t s);
 // unsorted: many particles were placed since the last sort (their order is emission order): the wider tile.
 int launch_p2g(const Dev& d, const Pass& p, const slosh_particle_t* particles, uint32_t n, bool unsorted, cudaStream_t s);
+// spread: the particles lie too far apart in their order for a CTA's tile (in placement order, or fewer than G2P_SPARSE a fluid cell).
+constexpr double G2P_SPARSE = 2.0;
 int launch_g2p(const Dev& d, const Pass& p, slosh_particle_t* particles, uint32_t n, const float* vel, const float* disp,
-               bool apply_density, bool unsorted, cudaStream_t s);
+               bool apply_density, bool spread, cudaStream_t s);
 // P2G as a per-brick gather (opt-in, SLOSH_P2G_GATHER=1): a per-cell particle index rebuilt every launch (counts
 // into cell_count with the rank of each particle in its cell, an exclusive scan, a scatter of particle ids), then
 // one CTA per active brick that visits the particles of the brick's cells and of the one-cell layer around it and

@@ -1096,13 +1096,15 @@ int launch_p2g_gather(const Dev& d, const Pass& p, const P2GGather& g, const slo
     return 4 + scans;
 }
 int launch_g2p(const Dev& d, const Pass& p, slosh_particle_t* particles, uint32_t n, const float* vel, const float* disp,
-               bool apply_density, bool unsorted, cudaStream_t s) {
+               bool apply_density, bool spread, cudaStream_t s) {
     if (n == 0) return 0;
     // Particles in no spatial order spread a CTA's box beyond the tile, and the pool is read after a search for the box:
     // 8.9 M of a 192^3 tank 1,876 us in random order and 549 in emission order, from the pool at once 1,641 and 498; of a
     // 128x128x96 tank 134 and 121 in emission order. The rule is P2G's; of particles that drift from a sort the tile stays ahead
-    // (192^3: 341 against 402 us a frame after the sort, 406 and 416 after 32, 480 and 486 after 64).
-    if (p.use_apic && !unsorted) {
+    // (192^3: 341 against 402 us a frame after the sort, 406 and 416 after 32, 480 and 486 after 64). Sorted particles spread so when
+    // a cell has few: all over 192^3 cells, tile and pool with the displacement, 0.25 a cell 160 and 144 us, 0.5 (1.3 a fluid cell) 291
+    // and 261, 1 (1.65) 488 and 490, 2 (2.4) 804 and 970; all over 64^3 cells 1 (1.7) 29.1 and 27.1, 2 (2.5) 43.4 both.
+    if (p.use_apic && !spread) {
         const int smem = (apply_density ? 6 : 3) * G2P_TILE_NODES * 4;
         auto kernel = apply_density ? k_g2p_tile<true> : k_g2p_tile<false>;
         kernel<<<(n + G2P_TILE_THREADS - 1u) / G2P_TILE_THREADS, G2P_TILE_THREADS, smem, s>>>(d, p, particles, n, vel, disp);

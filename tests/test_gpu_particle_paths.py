@@ -93,3 +93,30 @@ def test_apic_after_a_sort_matches_oracle(slosh, oracle_mod, count, order, speed
             assert not bad, bad
         g.end_frame()
         o.end_frame()
+
+
+# a sorted spray (fewer than two particles a fluid cell) takes the pool from its second frame on
+@pytest.mark.parametrize("density", [0, 1])
+def test_sorted_spray_matches_oracle(slosh, oracle_mod, density):
+    grid = (30, 24, 21)
+    s = slosh.settings_default()
+    s.grid_dim[:] = list(grid)
+    s.cell_size = 1.0 / max(grid)
+    s.particle_capacity = 16384
+    s.two_sided_density_projection = density
+    s.min_substeps = s.max_substeps = 1
+    s.sort_interval = 1
+    g, o = slosh.Simulation(s), oracle_mod.Oracle(s)
+    rec = _records(grid, 1200, "random", 3.0, 9)
+    for sim in (g, o):
+        sim.upload_particles(rec)
+    fi = A.frame_input(s, delta_time=1.0 / 120.0)
+    for _ in range(3):
+        assert g.begin_frame(fi) == o.begin_frame(fi)
+        g.substep(0)
+        o.substep(0)
+        bad = compare_state(g, o).failures()
+        assert not bad, bad
+        g.end_frame()
+        o.end_frame()
+        assert g.results().live_particles < 2 * g.results().fluid_cells
