@@ -5,7 +5,8 @@ import pytest
 from slosh_b200 import _abi as A
 from slosh_b200 import scenes
 
-from parity import compare_state, pair, run_frames
+from parity import pair, run_frames
+from parity import compare_state
 
 pytestmark = pytest.mark.gpu
 
